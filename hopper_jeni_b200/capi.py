@@ -7,11 +7,14 @@ symbol each header declares and the test-suite checks that the built libraries e
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _LIB = None
 _SELFTEST_LIB = None
+_BINDING = None
 
 GQA_OK = 0
 GQA_BWD_DETERMINISTIC = 1
@@ -112,6 +115,27 @@ def load_selftest_library():
             fn.argtypes = args
         _SELFTEST_LIB = lib
     return _SELFTEST_LIB
+
+
+def load_torch_binding():
+    """The native tensor-level host path (``_gqa_torch.so``: argument checks, allocation, autograd nodes), bound to the
+    functions of the library that :func:`load_library` found; raises if either has not been built."""
+    global _BINDING
+    if _BINDING is None:
+        lib = load_library()
+        path = os.path.join(_HERE, "_gqa_torch.so")
+        if not os.path.exists(path):
+            raise FileNotFoundError(f"{path} not found: build it with `python -m hopper_jeni_b200.build`")
+        import torch  # noqa: F401  (the module links against torch's libraries)
+
+        loader = importlib.machinery.ExtensionFileLoader("_gqa_torch", path)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_gqa_torch", path, loader=loader))
+        loader.exec_module(module)
+        module.bind(check, *(ctypes.cast(getattr(lib, fn), ctypes.c_void_p).value for fn in (
+            "gqa_fwd_ex", "gqa_bwd_ex", "gqa_bwd_workspace_bytes_ex", "gqa_fwd_varlen", "gqa_bwd_varlen",
+            "gqa_bwd_varlen_workspace_bytes")))
+        _BINDING = module
+    return _BINDING
 
 
 def check(fn: str, status: int) -> None:

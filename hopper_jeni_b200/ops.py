@@ -1,6 +1,7 @@
 """Tensor-level wrappers over the C ABI.
 
-torch is used only for device memory and streams; all arithmetic happens inside the library.
+torch is used only for device memory and streams; all arithmetic happens inside the library.  The operators' argument
+checks, allocations and launches run in the native binding (csrc/torch_binding.cpp).
 Layouts follow the reference launchers (src/attention/GQA_bwd_baseline.cu:549-554,
 src/attention/GQA_fwd_ref.cu:631-634): Q/O/dO/dQ ``[B,Hq,S,D]``, K/V/dK/dV ``[B,Hkv,S,D]`` bf16
 contiguous, LSE ``[B,Hq,S]`` fp32 (natural log).
@@ -19,6 +20,11 @@ def _stream_ptr(stream=None) -> int:
     return int(s.cuda_stream)
 
 
+def _stream_arg(stream):
+    """What the torch binding takes: None (the current stream of q's device) or the stream's handle."""
+    return None if stream is None else int(stream.cuda_stream)
+
+
 def _req(t: torch.Tensor, name: str, dtype) -> None:
     if not t.is_cuda:
         raise ValueError(f"{name} must be a CUDA tensor (this library has no CPU path)")
@@ -26,17 +32,6 @@ def _req(t: torch.Tensor, name: str, dtype) -> None:
         raise ValueError(f"{name} must be {dtype}, got {t.dtype}")
     if not t.is_contiguous():
         raise ValueError(f"{name} must be contiguous")
-
-
-def _req_like(t: torch.Tensor, name: str, like: torch.Tensor, shape=None, dtype=None) -> None:
-    """`t` must live on `like`'s device, be contiguous and have exactly the given shape and dtype: the C ABI
-    receives raw pointers, so a wrong-sized or wrong-device tensor would become an out-of-bounds access."""
-    _req(t, name, like.dtype if dtype is None else dtype)
-    if t.device != like.device:
-        raise ValueError(f"{name} is on {t.device}, expected {like.device}")
-    want = tuple(like.shape if shape is None else shape)
-    if tuple(t.shape) != want:
-        raise ValueError(f"{name} has shape {tuple(t.shape)}, expected {want}")
 
 
 def _dims(q, k, layout="bhsd"):
@@ -62,22 +57,7 @@ def gqa_forward(q, k, v, causal: bool = False, scale: float | None = None, out=N
                 layout: str = "bhsd"):
     """O, LSE = attention(Q, K, V).  Mirrors ``launch_gqa_v62`` with D and causal as arguments.
     ``layout="bshd"``: Q, K, V, O are [B,S,H,D] (``GQA_LAYOUT_BSHD``); LSE is [B,Hq,S] either way."""
-    lib = capi.load_library()
-    for t, n in ((q, "Q"), (k, "K"), (v, "V")):
-        _req(t, n, torch.bfloat16)
-    B, Hq, Hkv, S, D = _dims(q, k, layout)
-    scale = 1.0 / math.sqrt(D) if scale is None else float(scale)
-    out = torch.empty_like(q) if out is None else out
-    lse = torch.empty((B, Hq, S), dtype=torch.float32, device=q.device) if lse is None else lse
-    _req_like(v, "V", k)
-    _req_like(out, "O", q)
-    _req_like(lse, "LSE", q, shape=(B, Hq, S), dtype=torch.float32)
-    with torch.cuda.device(q.device):
-        rc = lib.gqa_fwd_ex(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(),
-                            B, Hq, Hkv, S, D, int(bool(causal)), scale, _stream_ptr(stream),
-                            capi.GQA_LAYOUT_BSHD if layout == "bshd" else 0)
-    capi.check("gqa_fwd_ex", rc)
-    return out, lse
+    return capi.load_torch_binding().forward(q, k, v, causal, scale, out, lse, _stream_arg(stream), layout)
 
 
 def bwd_workspace_bytes(B, Hq, Hkv, S, D, causal=False, split_heads: bool = False) -> int:
@@ -97,73 +77,18 @@ def gqa_backward(q, k, v, o, do, lse, causal: bool = False, scale: float | None 
     ``split_heads`` (``GQA_BWD_SPLIT_HEADS``): let a call with few KV tiles cut each tile's work over several thread
     blocks by query head (fp32 partial dK/dV, fixed-order sum); the workspace must be sized with the same option.
     ``dq_separate`` (``GQA_BWD_DQ_SEPARATE``): dQ from a separate query-parallel pass instead of the accumulator."""
-    lib = capi.load_library()
-    for t, n in ((q, "Q"), (k, "K"), (v, "V"), (o, "O"), (do, "dO")):
-        _req(t, n, torch.bfloat16)
-    _req(lse, "LSE", torch.float32)
-    B, Hq, Hkv, S, D = _dims(q, k, layout)
-    scale = 1.0 / math.sqrt(D) if scale is None else float(scale)
-    need = bwd_workspace_bytes(B, Hq, Hkv, S, D, causal, split_heads)
-    if need == 0:
-        capi.check("gqa_bwd_workspace_bytes", -2)
-    if workspace is None:
-        workspace = torch.empty(need, dtype=torch.uint8, device=q.device)
-    dq = torch.empty_like(q) if dq is None else dq
-    dk = torch.empty_like(k) if dk is None else dk
-    dv = torch.empty_like(v) if dv is None else dv
-    _req_like(v, "V", k)
-    for t, n in ((o, "O"), (do, "dO"), (dq, "dQ")):
-        _req_like(t, n, q)
-    for t, n in ((dk, "dK"), (dv, "dV")):
-        _req_like(t, n, k)
-    _req_like(lse, "LSE", q, shape=(B, Hq, S), dtype=torch.float32)
-    # its size is checked by the library (GQA_ERR_WORKSPACE, with the needed size in the error text)
-    if not workspace.is_cuda or workspace.device != q.device or not workspace.is_contiguous():
-        raise ValueError(f"workspace must be contiguous memory on {q.device}")
-    with torch.cuda.device(q.device):
-        args = (q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(),
-                dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, Hq, Hkv, S, D, int(bool(causal)), scale,
-                workspace.data_ptr(), workspace.numel() * workspace.element_size(), _stream_ptr(stream))
-        flags = ((capi.GQA_BWD_DETERMINISTIC if deterministic else 0) | (capi.GQA_LAYOUT_BSHD if layout == "bshd" else 0)
-                 | (capi.GQA_BWD_SPLIT_HEADS if split_heads else 0) | (capi.GQA_BWD_DQ_SEPARATE if dq_separate else 0))
-        rc = lib.gqa_bwd_ex(*args, flags) if flags else lib.gqa_bwd(*args)
-    capi.check("gqa_bwd_ex" if flags else "gqa_bwd", rc)
-    return dq, dk, dv
-
-
-def _packed_dims(q, k, cu_seqlens, max_seqlen):
-    """Shapes of a packed variable-length batch: q [T,Hq,D], k [T,Hkv,D], cu_seqlens int32 [n_seqs+1] on the device."""
-    if q.dim() != 3 or k.dim() != 3:
-        raise ValueError("packed batches are [total_tokens, H, D]")
-    T, Hq, D = q.shape
-    if k.shape[0] != T or k.shape[2] != D:
-        raise ValueError(f"K {tuple(k.shape)} does not match Q {tuple(q.shape)}")
-    if (cu_seqlens.dtype != torch.int32 or cu_seqlens.dim() != 1 or cu_seqlens.numel() < 2 or not cu_seqlens.is_cuda
-            or cu_seqlens.device != q.device or not cu_seqlens.is_contiguous()):
-        raise ValueError(f"cu_seqlens must be a contiguous int32 vector of n_seqs + 1 entries on {q.device}")
-    return T, Hq, k.shape[1], D, cu_seqlens.numel() - 1, int(max_seqlen)
+    flags = ((capi.GQA_BWD_DETERMINISTIC if deterministic else 0) | (capi.GQA_BWD_SPLIT_HEADS if split_heads else 0)
+             | (capi.GQA_BWD_DQ_SEPARATE if dq_separate else 0))
+    return capi.load_torch_binding().backward(q, k, v, o, do, lse, causal, scale, workspace, dq, dk, dv,
+                                              _stream_arg(stream), layout, flags)
 
 
 def gqa_forward_varlen(q, k, v, cu_seqlens, max_seqlen: int, causal: bool = False, scale: float | None = None,
                        out=None, lse=None, stream=None):
     """O [T,Hq,D] and LSE [Hq,T] of a packed variable-length batch (``gqa_fwd_varlen``): sequence i is the rows
     cu_seqlens[i] .. cu_seqlens[i+1]-1 of q [T,Hq,D] and k, v [T,Hkv,D] and attends only to itself."""
-    lib = capi.load_library()
-    for t, n in ((q, "Q"), (k, "K"), (v, "V")):
-        _req(t, n, torch.bfloat16)
-    T, Hq, Hkv, D, n_seqs, max_seqlen = _packed_dims(q, k, cu_seqlens, max_seqlen)
-    _req_like(v, "V", k)
-    scale = 1.0 / math.sqrt(D) if scale is None else float(scale)
-    out = torch.empty_like(q) if out is None else out
-    lse = torch.empty(Hq, T, dtype=torch.float32, device=q.device) if lse is None else lse
-    _req_like(out, "O", q)
-    _req_like(lse, "LSE", q, shape=(Hq, T), dtype=torch.float32)
-    with torch.cuda.device(q.device):
-        rc = lib.gqa_fwd_varlen(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(),
-                                cu_seqlens.data_ptr(), n_seqs, T, max_seqlen, Hq, Hkv, D, int(bool(causal)), scale,
-                                _stream_ptr(stream))
-    capi.check("gqa_fwd_varlen", rc)
-    return out, lse
+    return capi.load_torch_binding().forward_varlen(q, k, v, cu_seqlens, int(max_seqlen), causal, scale, out, lse,
+                                                    _stream_arg(stream))
 
 
 def bwd_varlen_workspace_bytes(total_tokens, Hq, Hkv, D) -> int:
@@ -173,35 +98,8 @@ def bwd_varlen_workspace_bytes(total_tokens, Hq, Hkv, D) -> int:
 def gqa_backward_varlen(q, k, v, o, do, lse, cu_seqlens, max_seqlen: int, causal: bool = False,
                         scale: float | None = None, workspace=None, dq=None, dk=None, dv=None, stream=None):
     """dQ, dK, dV of a packed variable-length batch (``gqa_bwd_varlen``); tensors as in gqa_forward_varlen."""
-    lib = capi.load_library()
-    for t, n in ((q, "Q"), (k, "K"), (v, "V"), (o, "O"), (do, "dO")):
-        _req(t, n, torch.bfloat16)
-    _req(lse, "LSE", torch.float32)
-    T, Hq, Hkv, D, n_seqs, max_seqlen = _packed_dims(q, k, cu_seqlens, max_seqlen)
-    scale = 1.0 / math.sqrt(D) if scale is None else float(scale)
-    need = bwd_varlen_workspace_bytes(T, Hq, Hkv, D)
-    if need == 0:
-        capi.check("gqa_bwd_varlen_workspace_bytes", -2)
-    if workspace is None:
-        workspace = torch.empty(need, dtype=torch.uint8, device=q.device)
-    dq = torch.empty_like(q) if dq is None else dq
-    dk = torch.empty_like(k) if dk is None else dk
-    dv = torch.empty_like(v) if dv is None else dv
-    _req_like(v, "V", k)
-    for t, n in ((o, "O"), (do, "dO"), (dq, "dQ")):
-        _req_like(t, n, q)
-    for t, n in ((dk, "dK"), (dv, "dV")):
-        _req_like(t, n, k)
-    _req_like(lse, "LSE", q, shape=(Hq, T), dtype=torch.float32)
-    if not workspace.is_cuda or workspace.device != q.device or not workspace.is_contiguous():
-        raise ValueError(f"workspace must be contiguous memory on {q.device}")
-    with torch.cuda.device(q.device):
-        rc = lib.gqa_bwd_varlen(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(),
-                                dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), cu_seqlens.data_ptr(), n_seqs, T,
-                                max_seqlen, Hq, Hkv, D, int(bool(causal)), scale, workspace.data_ptr(),
-                                workspace.numel() * workspace.element_size(), _stream_ptr(stream))
-    capi.check("gqa_bwd_varlen", rc)
-    return dq, dk, dv
+    return capi.load_torch_binding().backward_varlen(q, k, v, o, do, lse, cu_seqlens, int(max_seqlen), causal, scale,
+                                                     workspace, dq, dk, dv, _stream_arg(stream))
 
 
 def bwd_stage_times(q, k, v, o, do, lse, causal, scale, workspace, dq, dk, dv, flush=None):
