@@ -1022,20 +1022,6 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     }
 }
 
-// Thread blocks of the main kernel that run at the same time: one per SM (shared memory and TMEM allow no second).
-int resident_blocks() {
-    static thread_local int cached_dev = -1, cached = 0;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 1;
-    if (dev != cached_dev) {
-        int sms = 0;
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) return 1;
-        cached = sms;
-        cached_dev = dev;
-    }
-    return cached;
-}
-
 // Causal order: how many (batch, KV head) groups form a super-group (the list runs super-group by super-group, KV
 // tile by KV tile inside, longest items first).  Few groups at a time means many KV tiles of the same group in
 // flight together, all streaming that group's Q/dO tiles through L2 at nearly the same time, so HBM is read fewer
@@ -1107,10 +1093,11 @@ int launch_bwd_t(const void* Q, const void* K, const void* V, const void* dO, co
     p.scale = s.scale;
     p.scale_log2 = s.scale * 1.4426950408889634f;
     p.groups = (varlen ? s.n_seqs : s.B) * s.Hkv;
-    p.sg = dq_turn ? p.groups : causal_super_group(p.groups, p.n_tiles, resident_blocks());
+    p.sg = dq_turn ? p.groups : causal_super_group(p.groups, p.n_tiles, sm_count());
     p.n_items = p.n_tiles * p.groups * parts;
-    // persistent, except in the deterministic mode (see the work-item comment in the kernel)
-    const unsigned grid = (unsigned)(dq_turn ? p.n_items : std::min(p.n_items, resident_blocks()));
+    // persistent, one block per SM (shared memory and TMEM allow no second), except in the deterministic mode (see the
+    // work-item comment in the kernel)
+    const unsigned grid = (unsigned)(dq_turn ? p.n_items : std::min(p.n_items, sm_count()));
     kernel<<<grid, Cfg::kThreads, Cfg::kSmemTotal, stream>>>(mq, mk, mv, mdo, mdq, mlse, mdlt, p);
     count_launch();
     GQA_CUDA_TRY(cudaGetLastError());

@@ -41,6 +41,9 @@ int make_tile3_tmap(CUtensorMap* out, const void* base, uint64_t cols, uint64_t 
 int make_f32box3_tmap(CUtensorMap* out, const void* base, uint64_t cols, uint64_t S, uint64_t n_outer, uint32_t box_rows);
 int make_col8_3_tmap(CUtensorMap* out, const void* base, uint64_t S, uint64_t n_outer, uint32_t box_rows);
 
+// SMs of the current device (1 when it cannot be asked).
+int sm_count();
+
 // Device word that forward kernels report bounded-wait failures into (per device).
 int forward_status_word(unsigned int** out);
 

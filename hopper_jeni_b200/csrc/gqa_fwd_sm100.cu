@@ -1,10 +1,11 @@
 // GQA forward for sm_100a: O = softmax(scale * Q K^T [+ causal]) V, LSE.
 //
-// One CTA owns two 128-row query tiles of one (batch, query head) and streams the
-// KV head's 128-row key/value blocks through a TMA ring.  Roles:
+// A work item is two 128-row query tiles (one, where every tile gets an SM of its own) of one (batch, query
+// head); the KV head's 128-row key/value blocks stream through a TMA ring.  A thread block works through
+// several items (see the work-item comment).  Roles:
 //   warps 0-3  softmax warpgroup for query tile 0 (thread = query row = TMEM lane)
 //   warps 4-7  softmax warpgroup for query tile 1
-//   warp  8    TMA producer (Q once, K and V rings)
+//   warp  8    TMA producer (Q once per item, K and V rings) and taker of further items
 //   warps 9,10 UMMA issuers, one per query tile: S = Q K^T and O += P V (P read from TMEM)
 // Every key block is handled as two half-blocks of 64 keys, and the 128 fp32 S columns of a tile are two
 // 64-column buffers: while the softmax warpgroup works on half-block j, the issuer has already produced
@@ -45,6 +46,7 @@ constexpr int kPanel = kTile * 128;    // bytes of one 64-column panel of a 128-
 constexpr int kHalf = 64;               // keys per half-block
 constexpr int kFwdThreads = 352;
 constexpr int kWarpTma = 8, kWarpMma0 = 9;
+constexpr int kItemSlots = 2;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kRescaleThreshold = 8.0f;  // in log2 units
@@ -69,8 +71,9 @@ struct FwdParams {
     __nv_bfloat16* O;
     float* LSE;
     unsigned int* status;
-    int Hq, Hkv, S, causal, n_pairs, bshd;
-    const int* cu;     // packed variable-length batch: sequence starts (blockIdx.z = sequence), else null
+    int Hq, Hkv, S, causal, bshd;
+    int tiles, n_groups;  // query tiles per item (1 or 2), items per (sequence, query head)
+    const int* cu;     // packed variable-length batch: sequence starts (z of an item = sequence), else null
     int d_real;        // head dimension of the tensors (<= D of the kernel; the columns beyond it read as zeros)
     float scale_log2;  // scale * log2(e)
 };
@@ -98,41 +101,71 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     uint64_t* k_empty = k_full + Cfg::kStages;     // [kStages]
     uint64_t* v_full = k_empty + Cfg::kStages;     // [kStages]
     uint64_t* v_empty = v_full + Cfg::kStages;     // [kStages]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(v_empty + Cfg::kStages);
+    uint64_t* q_empty = v_empty + Cfg::kStages;    // [2]  per tile: the last S of the item has been computed
+    uint64_t* o_empty = q_empty + 2;               // [2]  per tile: the epilogue has read O
+    uint64_t* item_full = o_empty + 2;             // [kItemSlots] producer -> everybody: the block's next item
+    uint64_t* item_empty = item_full + kItemSlots; // [kItemSlots]
+    uint64_t* clc_full = item_empty + kItemSlots;  // answer to a request for another item
+    uint8_t* clc_answer = reinterpret_cast<uint8_t*>(clc_full + 2);
+    constexpr int kBars = 16 + 4 * Cfg::kStages + 4 + 2 * kItemSlots + 2;
+    static_assert(kBars % 2 == 0, "the answer is 16-byte aligned");
+    volatile int* item_slot = reinterpret_cast<volatile int*>(clc_answer + 16);  // [kItemSlots][4]: x, y, z of the block
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(clc_answer + 16 + kItemSlots * 16);
     volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(tmem_slot + 1);
+    static_assert(kBars * 8 + 16 + kItemSlots * 16 + 8 <= Cfg::kBarBytes, "barrier area");
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int lane = tid & 31;
     AbortCtx ctx{abort_flag, p.status};
 
-    // ---- work decode ------------------------------------------------------------
-    const int pair = p.causal ? (p.n_pairs - 1 - (int)blockIdx.x) : (int)blockIdx.x;  // heavy causal tiles first
-    const int hq = blockIdx.y;
-    const int hkv = hq / (p.Hq / p.Hkv);
-    const int q0 = pair * 2 * kTile;
+    // ---- work items.  An item is what one thread block of the grid stands for: `tiles` query tiles of one query head.
+    // A block works through its own item and then takes over blocks of the same launch that have not started yet, one
+    // after the other (cluster launch control hands them out in grid order), with every ring and barrier carrying on:
+    // the next item's Q, K and V are loaded and its first S is computed while the last products and the epilogue of the
+    // one before run, and the set-up of a block is paid once per SM.  One block per item cost about 12 000 cycles of
+    // start and finish per item.  B200, back to back: B16 Hq16 S2048 D64 414 -> 380 us (804 -> 703 thousand SM cycles),
+    // S1024 136 -> 116 us, causal B8 Hq12 S4096 380 -> 343 us; D = 128, where the power cap sets the clock, 1 to 2 %
+    // (B16 Hq16 S4096 1 940 -> 1 904 us); a launch of one item per SM is unchanged.  The same loop without the take-over
+    // is as slow as before (412 us), so it is the overlap that pays.
+    struct Item {
+        int hq, q0, b, y0, len, n_tiles;
+        int n_blk0, n_blk1, n_max;  // key blocks of the two tiles and the larger of the two
+    };
     // Packed variable-length batch: the sequence is a row range [y0, y0 + len) of the one [T, H*D] matrix; rows past
     // its end belong to the next sequence (or read as zeros past T): as keys they are masked like keys beyond S,
-    // as queries they are computed and not stored.  The grid covers max_seqlen: blocks beyond this sequence leave
-    // here, before anything is set up.
-    int b = blockIdx.z, y0 = 0, len = p.S;
-    if (p.cu) {
-        y0 = p.cu[b];
-        len = p.cu[b + 1] - y0;
-        b = 0;
-        if (q0 >= len) return;
-    }
-    const int n_tiles = (q0 + kTile < len) ? 2 : 1;
-    const int n_blocks_all = (len + kTile - 1) / kTile;  // the last block may be partial: keys at and beyond len are masked
-    int n_blk[2];
-    n_blk[0] = p.causal ? (q0 / kTile + 1) : n_blocks_all;
-    n_blk[1] = (n_tiles == 2) ? (p.causal ? (q0 / kTile + 2) : n_blocks_all) : 0;
-    const int n_max = n_blk[1] > n_blk[0] ? n_blk[1] : n_blk[0];
-    const int q_row0 = (b * p.Hq + hq) * p.S + y0 + q0;   // row in [B,Hq,S] order (LSE)
-    // Tensor-map coordinates (x = column, y = position in the sequence, z = matrix).  [B,H,S,D] is B*H matrices
-    // [S, D]; [B,S,H,D] is B matrices [S, H*D] with the head at x = head * D.  Rows at y >= S read as zeros.
-    const int q_x = p.bshd ? hq * D : 0, q_z = p.bshd ? b : b * p.Hq + hq;
-    const int kv_x = p.bshd ? hkv * D : 0, kv_z = p.bshd ? b : b * p.Hkv + hkv;
+    // as queries they are computed and not stored.  The grid covers max_seqlen: an item beyond its sequence has
+    // n_tiles = 0 and is passed over by the producer.
+    auto decode = [&](int x, int y, int z) -> Item {
+        Item w;
+        const int idx = p.causal ? (p.n_groups - 1 - x) : x;  // heavy causal tiles first
+        w.hq = y;
+        w.q0 = idx * p.tiles * kTile;
+        w.b = z;
+        w.y0 = 0;
+        w.len = p.S;
+        if (p.cu) {
+            w.y0 = p.cu[z];
+            w.len = p.cu[z + 1] - w.y0;
+            w.b = 0;
+        }
+        w.n_tiles = w.q0 >= w.len ? 0 : (p.tiles == 2 && w.q0 + kTile < w.len) ? 2 : 1;
+        const int n_blocks_all = (w.len + kTile - 1) / kTile;  // the last block may be partial: keys at and beyond len are masked
+        w.n_blk0 = p.causal ? (w.q0 / kTile + 1) : n_blocks_all;
+        w.n_blk1 = (w.n_tiles == 2) ? (p.causal ? (w.q0 / kTile + 2) : n_blocks_all) : 0;
+        w.n_max = max(w.n_blk0, w.n_blk1);
+        return w;
+    };
+    // The j-th item of this block, published by the producer: false = no more (or give up).
+    auto fetch_item = [&](int j, Item& w) -> bool {
+        const int sl = j % kItemSlots;
+        if (!mbar_wait(&item_full[sl], (j / kItemSlots) & 1, ctx, 14)) return false;
+        const int x = item_slot[sl * 4 + 0], y = item_slot[sl * 4 + 1], z = item_slot[sl * 4 + 2];
+        mbar_arrive(&item_empty[sl]);
+        if (x < 0) return false;
+        w = decode(x, y, z);
+        return true;
+    };
 
     // ---- setup ------------------------------------------------------------------
     if (tid == 0) {
@@ -141,7 +174,9 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
         *abort_flag = (*reinterpret_cast<volatile unsigned int*>(p.status) != 0u) ? 98u : 0u;
         for (int i = 0; i < 2; ++i) {
             mbar_init(&q_full[i], 1);
+            mbar_init(&q_empty[i], 1);
             mbar_init(&o_full[i], 1);
+            mbar_init(&o_empty[i], 128);
         }
         for (int i = 0; i < 4; ++i) {
             mbar_init(&s_full[i], 1);
@@ -150,10 +185,15 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
         }
         for (int i = 0; i < Cfg::kStages; ++i) {
             mbar_init(&k_full[i], 1);
-            mbar_init(&k_empty[i], n_tiles);  // one commit per issuer that uses the block
+            mbar_init(&k_empty[i], 2);  // both issuers release every block, also one they do not use
             mbar_init(&v_full[i], 1);
-            mbar_init(&v_empty[i], n_tiles);
+            mbar_init(&v_empty[i], 2);
         }
+        for (int i = 0; i < kItemSlots; ++i) {
+            mbar_init(&item_full[i], 1);
+            mbar_init(&item_empty[i], 320);  // every softmax and issuer thread
+        }
+        mbar_init(clc_full, 1);
         fence_mbar_init();
     }
     if (warp == kWarpMma0) {
@@ -175,96 +215,170 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
             tma_prefetch_desc(&mapQ);
             tma_prefetch_desc(&mapK);
             tma_prefetch_desc(&mapV);
-            for (int t = 0; t < n_tiles; ++t) {
-                mbar_expect_tx(&q_full[t], Cfg::kTileBytes);
-                for (int pn = 0; pn < Cfg::kPanels; ++pn)
-                    tma_load_3d(sQ + t * Cfg::kTileBytes + pn * kPanel, &mapQ, &q_full[t], q_x + pn * 64, y0 + q0 + t * kTile, q_z);
-            }
-            for (int n = 0; n < n_max; ++n) {
-                const int st = n % Cfg::kStages;
-                const uint32_t use = n / Cfg::kStages;
-                if (use > 0 && !mbar_wait(&k_empty[st], (use - 1) & 1, ctx, 10)) break;
-                mbar_expect_tx(&k_full[st], Cfg::kTileBytes);
-                for (int pn = 0; pn < Cfg::kPanels; ++pn)
-                    tma_load_3d(sK + st * Cfg::kTileBytes + pn * kPanel, &mapK, &k_full[st], kv_x + pn * 64, y0 + n * kTile, kv_z);
-                if (use > 0 && !mbar_wait(&v_empty[st], (use - 1) & 1, ctx, 11)) break;
-                mbar_expect_tx(&v_full[st], Cfg::kTileBytes);
-                for (int pn = 0; pn < Cfg::kPanels; ++pn)
-                    tma_load_3d(sV + st * Cfg::kTileBytes + pn * kPanel, &mapV, &v_full[st], kv_x + pn * 64, y0 + n * kTile, kv_z);
+            uint32_t n_claims = 0;
+            int x = blockIdx.x, y = blockIdx.y, z = blockIdx.z;
+            // The next item that has work: x = -1 when there is none.  False: a wait gave up.
+            auto claim = [&]() -> bool {
+                for (;;) {
+                    mbar_expect_tx(clc_full, 16);
+                    clc_try_cancel(clc_answer, clc_full);
+                    if (!mbar_wait(clc_full, n_claims & 1, ctx, 15)) return false;
+                    ++n_claims;
+                    const bool taken = clc_read_answer(clc_answer, x, y, z);
+                    fence_proxy_async_smem();  // the answer has been read before the next one is written
+                    if (!taken) {
+                        x = -1;
+                        return true;
+                    }
+                    if (!p.cu || decode(x, y, z).n_tiles > 0) return true;
+                }
+            };
+            bool ok = true;
+            if (p.cu && decode(x, y, z).n_tiles == 0) ok = claim();
+            uint32_t kb = 0;             // key blocks loaded so far, over all items
+            int n_q[2] = {0, 0};         // loads of the two Q tiles so far
+            for (int j = 0; ok; ++j) {
+                const int sl = j % kItemSlots;
+                if (j >= kItemSlots && !mbar_wait(&item_empty[sl], (j / kItemSlots - 1) & 1, ctx, 13)) break;
+                // a block of this launch that gave up has left a non-zero status word: stop taking items
+                if (j > 0 && *reinterpret_cast<volatile unsigned int*>(p.status) != 0u) {
+                    *abort_flag = 98u;
+                    break;
+                }
+                item_slot[sl * 4 + 0] = x;
+                item_slot[sl * 4 + 1] = y;
+                item_slot[sl * 4 + 2] = z;
+                mbar_arrive(&item_full[sl]);
+                if (x < 0) break;
+                const Item w = decode(x, y, z);
+                const int hkv = w.hq / (p.Hq / p.Hkv);
+                // Tensor-map coordinates (x = column, y = position in the sequence, z = matrix).  [B,H,S,D] is B*H matrices
+                // [S, D]; [B,S,H,D] is B matrices [S, H*D] with the head at x = head * D.  Rows at y >= S read as zeros.
+                const int q_x = p.bshd ? w.hq * D : 0, q_z = p.bshd ? w.b : w.b * p.Hq + w.hq;
+                const int kv_x = p.bshd ? hkv * D : 0, kv_z = p.bshd ? w.b : w.b * p.Hkv + hkv;
+                for (int t = 0; t < w.n_tiles && ok; ++t) {
+                    if (n_q[t] > 0 && !mbar_wait(&q_empty[t], (n_q[t] - 1) & 1, ctx, 12)) { ok = false; break; }
+                    ++n_q[t];
+                    mbar_expect_tx(&q_full[t], Cfg::kTileBytes);
+                    for (int pn = 0; pn < Cfg::kPanels; ++pn)
+                        tma_load_3d(sQ + t * Cfg::kTileBytes + pn * kPanel, &mapQ, &q_full[t], q_x + pn * 64, w.y0 + w.q0 + t * kTile, q_z);
+                }
+                for (int n = 0; n < w.n_max && ok; ++n, ++kb) {
+                    const uint32_t st = kb % Cfg::kStages;
+                    const uint32_t use = kb / Cfg::kStages;
+                    if (use > 0 && !mbar_wait(&k_empty[st], (use - 1) & 1, ctx, 10)) { ok = false; break; }
+                    mbar_expect_tx(&k_full[st], Cfg::kTileBytes);
+                    for (int pn = 0; pn < Cfg::kPanels; ++pn)
+                        tma_load_3d(sK + st * Cfg::kTileBytes + pn * kPanel, &mapK, &k_full[st], kv_x + pn * 64, w.y0 + n * kTile, kv_z);
+                    if (use > 0 && !mbar_wait(&v_empty[st], (use - 1) & 1, ctx, 11)) { ok = false; break; }
+                    mbar_expect_tx(&v_full[st], Cfg::kTileBytes);
+                    for (int pn = 0; pn < Cfg::kPanels; ++pn)
+                        tma_load_3d(sV + st * Cfg::kTileBytes + pn * kPanel, &mapV, &v_full[st], kv_x + pn * 64, w.y0 + n * kTile, kv_z);
+                }
+                if (ok) ok = claim();
             }
         }
     } else if (warp >= kWarpMma0) {
         // ======================= issuer of tile t: S(j) = Q K(j)^T per half-block, O += P(j) V(j) =======================
         // The whole warp runs the loop (uniform control flow); `leader` marks the one lane that issues.
         const int t = warp - kWarpMma0;
-        if (t < n_tiles) {
-            const uint32_t leader = elect_one() ? 1u : 0u;
-            const uint32_t idesc_qk = make_idesc_bf16(128, kHalf, false, false);
-            const uint32_t idesc_pv = make_idesc_bf16(128, D, false, true);
-            const uint32_t q_addr = smem_u32(sQ) + t * Cfg::kTileBytes, k_addr = smem_u32(sK), v_addr = smem_u32(sV);
-            const uint32_t colS = tmem + (t ? Cfg::kColS1 : Cfg::kColS0), colO = tmem + (t ? Cfg::kColO1 : Cfg::kColO0);
-            const int total = 2 * n_blk[t];
-            bool ok = mbar_wait(&q_full[t], 0, ctx, 20);
-            // S(j): rows 64h.. of key block n = j/2 are the B operand (K-major panels, 64 rows = 8192 bytes down)
-            auto issue_qk = [&](int j) -> bool {
-                const int n = j >> 1, h = j & 1, st = n % Cfg::kStages;
-                if (h == 0 && !mbar_wait(&k_full[st], (n / Cfg::kStages) & 1, ctx, 21)) return false;
-                tc_fence_after_sync();
-                const uint32_t b0 = k_addr + st * Cfg::kTileBytes + h * (kHalf * 128);
+        const uint32_t leader = elect_one() ? 1u : 0u;
+        const uint32_t idesc_qk = make_idesc_bf16(128, kHalf, false, false);
+        const uint32_t idesc_pv = make_idesc_bf16(128, D, false, true);
+        const uint32_t q_addr = smem_u32(sQ) + t * Cfg::kTileBytes, k_addr = smem_u32(sK), v_addr = smem_u32(sV);
+        const uint32_t colS = tmem + (t ? Cfg::kColS1 : Cfg::kColS0), colO = tmem + (t ? Cfg::kColO1 : Cfg::kColO0);
+        bool ok = true;
+        // running counts over all items of this block (ring stages and barrier parities): key blocks of the rings,
+        // key blocks and items of this tile
+        uint32_t kb = 0, cb = 0, n_done = 0;
+        Item w;
+        for (int it = 0; ok && fetch_item(it, w); ++it) {
+            const uint32_t n_blk = t ? w.n_blk1 : w.n_blk0, n_max = w.n_max;
+            if (n_blk > 0) {
+                ok = mbar_wait(&q_full[t], n_done & 1, ctx, 20);
+                // S of half h of key block n: rows 64h.. of the block are the B operand (K-major panels, 64 rows = 8192
+                // bytes down).  It goes where P of the same half of the block before lives: that product must have completed.
+                auto issue_qk = [&](uint32_t n, uint32_t h) -> bool {
+                    const uint32_t st = (kb + n) % Cfg::kStages;
+                    if (cb + n > 0 && !mbar_wait(&pv_done[t * 2 + h], (cb + n - 1) & 1, ctx, 22)) return false;
+                    if (h == 0 && !mbar_wait(&k_full[st], ((kb + n) / Cfg::kStages) & 1, ctx, 21)) return false;
+                    tc_fence_after_sync();
+                    const uint32_t b0 = k_addr + st * Cfg::kTileBytes + h * (kHalf * 128);
 #pragma unroll
-                for (int kk = 0; kk < D / 16; ++kk) {
-                    const uint32_t off = (kk >> 2) * kPanel + (kk & 3) * 32;
-                    umma_ss_pred(leader, colS + h * kHalf, make_sdesc_sw128(q_addr + off, 16, 1024),
-                                 make_sdesc_sw128(b0 + off, 16, 1024), idesc_qk, kk > 0);
-                }
-                umma_commit_pred(leader, &s_full[t * 2 + h]);
-                if (h == 1) umma_commit_pred(leader, &k_empty[st]);
-                if (t == 0) GQA_FTRACE(1, j, 0);
-                return true;
-            };
-            if (ok) ok = issue_qk(0);
-            for (int j = 0; j < total && ok; ++j) {
-                const int n = j >> 1, h = j & 1, st = n % Cfg::kStages;
-                if (j + 1 < total) {
-                    // S(j+1) goes where P(j-1) lives: that product must have completed
-                    if (j >= 1) ok = mbar_wait(&pv_done[t * 2 + (h ^ 1)], ((j - 1) >> 1) & 1, ctx, 22);
-                    if (ok) ok = issue_qk(j + 1);
-                    if (!ok) break;
-                }
-                if (h == 0) ok = mbar_wait(&v_full[st], (n / Cfg::kStages) & 1, ctx, 23);
-                if (ok) ok = mbar_wait(&p_full[t * 2 + h], n & 1, ctx, 24);
-                if (!ok) break;
-                tc_fence_after_sync();
-                if (t == 0) GQA_FTRACE(1, j, 1);
-                const uint32_t b0 = v_addr + st * Cfg::kTileBytes + h * (kHalf / 16) * 2048;
+                    for (int kk = 0; kk < D / 16; ++kk) {
+                        const uint32_t off = (kk >> 2) * kPanel + (kk & 3) * 32;
+                        umma_ss_pred(leader, colS + h * kHalf, make_sdesc_sw128(q_addr + off, 16, 1024),
+                                     make_sdesc_sw128(b0 + off, 16, 1024), idesc_qk, kk > 0);
+                    }
+                    umma_commit_pred(leader, &s_full[t * 2 + h]);
+                    if (h == 1) umma_commit_pred(leader, &k_empty[st]);
+                    if (h == 1 && n + 1 == n_blk) umma_commit_pred(leader, &q_empty[t]);
+                    if (t == 0) GQA_FTRACE(1, 2 * n + h, 0);
+                    return true;
+                };
+                if (ok) ok = issue_qk(0, 0);
+#pragma unroll 1
+                for (uint32_t n = 0; n < n_blk && ok; ++n) {
+                    const uint32_t st = (kb + n) % Cfg::kStages;
 #pragma unroll
-                for (int kk = 0; kk < kHalf / 16; ++kk)
-                    umma_ts_pred(leader, colO, colS + h * kHalf + kk * 8, make_sdesc_sw128(b0 + kk * 2048, kPanel, 1024),
-                                 idesc_pv, (j > 0 || kk > 0));
-                umma_commit_pred(leader, &pv_done[t * 2 + h]);
-                if (h == 1) umma_commit_pred(leader, &v_empty[st]);
-                if (j + 1 == total) umma_commit_pred(leader, &o_full[t]);
-                if (t == 0) GQA_FTRACE(1, j, 2);
+                    for (uint32_t h = 0; h < 2; ++h) {
+                        if (ok && (h == 0 || n + 1 < n_blk)) ok = issue_qk(n + h, h ^ 1);  // the next S
+                        if (ok && h == 0) ok = mbar_wait(&v_full[st], ((kb + n) / Cfg::kStages) & 1, ctx, 23);
+                        if (ok && h == 0 && n == 0 && n_done > 0) ok = mbar_wait(&o_empty[t], (n_done - 1) & 1, ctx, 25);  // the item before has read O
+                        if (ok) ok = mbar_wait(&p_full[t * 2 + h], (cb + n) & 1, ctx, 24);
+                        if (!ok) break;
+                        tc_fence_after_sync();
+                        if (t == 0) GQA_FTRACE(1, 2 * n + h, 1);
+                        const uint32_t b0 = v_addr + st * Cfg::kTileBytes + h * (kHalf / 16) * 2048;
+#pragma unroll
+                        for (int kk = 0; kk < kHalf / 16; ++kk)
+                            umma_ts_pred(leader, colO, colS + h * kHalf + kk * 8, make_sdesc_sw128(b0 + kk * 2048, kPanel, 1024),
+                                         idesc_pv, (n > 0 || h > 0 || kk > 0));
+                        umma_commit_pred(leader, &pv_done[t * 2 + h]);
+                        if (h == 1) umma_commit_pred(leader, &v_empty[st]);
+                        if (h == 1 && n + 1 == n_blk) umma_commit_pred(leader, &o_full[t]);
+                        if (t == 0) GQA_FTRACE(1, 2 * n + h, 2);
+                    }
+                }
+                ++n_done;
             }
+            // blocks that only the other tile uses: released as soon as they are there (waited for, so that the arrival
+            // falls into the right phase)
+            for (uint32_t n = n_blk; n < n_max && ok; ++n) {
+                const uint32_t st = (kb + n) % Cfg::kStages;
+                const uint32_t par = ((kb + n) / Cfg::kStages) & 1;
+                ok = mbar_wait(&k_full[st], par, ctx, 26);
+                if (ok && leader) mbar_arrive(&k_empty[st]);
+                if (ok) ok = mbar_wait(&v_full[st], par, ctx, 27);
+                if (ok && leader) mbar_arrive(&v_empty[st]);
+            }
+            kb += n_max;
+            cb += n_blk;
         }
     } else {
         // ======================= softmax warpgroups =======================
         const int t = warp >> 2;                      // query tile owned by this warpgroup
         const int r = (warp & 3) * 32 + lane;         // row inside the tile == TMEM lane
-        if (t < n_tiles) {
+        uint32_t cb = 0, n_done = 0;                  // key blocks and items of this tile so far (barrier parities)
+        bool ok = true;
+        Item w;
+        for (int it = 0; ok && fetch_item(it, w); ++it) {
+            const int n_blk = t ? w.n_blk1 : w.n_blk0;
+            if (n_blk == 0) continue;
+            const int q0 = w.q0, len = w.len, hq = w.hq, b = w.b, y0 = w.y0;
+            const int q_row0 = (b * p.Hq + hq) * p.S + y0 + q0;   // row in [B,Hq,S] order (LSE)
             const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
             const uint32_t tS = tmem + lane_addr + (t == 0 ? Cfg::kColS0 : Cfg::kColS1);
             const uint32_t tO = tmem + lane_addr + (t == 0 ? Cfg::kColO0 : Cfg::kColO1);
             const float c = p.scale_log2;
             const uint64_t c2 = pack_f32x2(c, c);
-            const int total = 2 * n_blk[t];
+            const int total = 2 * n_blk;
             const int diag_block = (q0 + t * kTile) / kTile;  // only this block needs the causal mask
             float m_run = -INFINITY;  // running maximum of the raw logits that P is measured against
             float l_run = 0.f;
-            bool ok = true;
             for (int j = 0; j < total; ++j) {
                 const int n = j >> 1, h = j & 1;
-                ok = mbar_wait(&s_full[t * 2 + h], n & 1, ctx, 30);
+                ok = mbar_wait(&s_full[t * 2 + h], (cb + n) & 1, ctx, 30);
                 if (!ok) break;
                 tc_fence_after_sync();
                 if (warp == 0) GQA_FTRACE(0, j, 0);
@@ -306,7 +420,7 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                     m_run = m_next;
                     if (j > 0) {
                         // O holds P(0..j-1) V; the last of those products may still be running
-                        ok = mbar_wait(&pv_done[t * 2 + (h ^ 1)], ((j - 1) >> 1) & 1, ctx, 32);
+                        ok = mbar_wait(&pv_done[t * 2 + (h ^ 1)], (cb + ((j - 1) >> 1)) & 1, ctx, 32);
                         if (!ok) break;
                         tc_fence_after_sync();
 #pragma unroll 1
@@ -374,7 +488,7 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                 GQA_FTRACE(t == 0 ? 3 : 5, j, warp & 3);
             }
             // epilogue: O / l -> bf16, LSE
-            if (ok) ok = mbar_wait(&o_full[t], 0, ctx, 31);
+            if (ok) ok = mbar_wait(&o_full[t], n_done & 1, ctx, 31);
             if (ok) {
                 tc_fence_after_sync();
                 // rows beyond the end of the sequence are not stored (the TMEM loads below are warp-wide
@@ -400,7 +514,12 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                     }
                 }
                 if (p.LSE && row_ok) p.LSE[grow_] = (m_run * c + log2f(l_run)) * kLn2;
+                // every column of O has been read: the next item's first product may overwrite them
+                tc_fence_before_sync();
+                mbar_arrive(&o_empty[t]);
             }
+            cb += n_blk;
+            ++n_done;
         }
     }
 
@@ -441,9 +560,14 @@ int launch_fwd_t(const void* Q, const void* K, const void* V, void* O, float* LS
     p.bshd = s.bshd;
     p.d_real = s.D;
     p.cu = s.cu_seqlens;
-    p.n_pairs = ((s.cu_seqlens ? s.max_seqlen : s.S) + 2 * kTile - 1) / (2 * kTile);
+    // Two query tiles per item share the K/V blocks and keep the tensor core busy in turns; one tile per item finishes
+    // sooner when every tile gets an SM of its own.  B200, D = 128 causal: 128 tiles (B1 Hq16 S1024) 22.5 us as single
+    // tiles against 25.6 us as pairs; 192 tiles (B2 Hq12 S1000) 30.8 against 26.6: the second round costs more.
+    const int n_tiles = ((s.cu_seqlens ? s.max_seqlen : s.S) + kTile - 1) / kTile, n_seqs = s.cu_seqlens ? s.n_seqs : s.B;
+    p.tiles = (long long)n_tiles * s.Hq * n_seqs <= sm_count() ? 1 : 2;
+    p.n_groups = (n_tiles + p.tiles - 1) / p.tiles;
     p.scale_log2 = s.scale * kLog2e;
-    dim3 grid(p.n_pairs, s.Hq, s.cu_seqlens ? s.n_seqs : s.B);
+    dim3 grid(p.n_groups, s.Hq, n_seqs);
     gqa_fwd_sm100_kernel<D><<<grid, kFwdThreads, Cfg::kSmemTotal, stream>>>(mq, mk, mv, p);
     count_launch();
     GQA_CUDA_TRY(cudaGetLastError());

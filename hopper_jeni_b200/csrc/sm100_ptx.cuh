@@ -162,6 +162,35 @@ __device__ __forceinline__ void st_release_gpu(unsigned int* p, unsigned int v) 
 }
 
 // ----------------------------------------------------------------------------
+// Cluster launch control: a running thread block takes over a block of its own launch that has not started yet.
+// The request is asynchronous; its 16-byte answer lands in shared memory (16-byte aligned) and completes 16 bytes of
+// transactions on the mbarrier.  After an answer "nothing left" no further request may be made.
+// ----------------------------------------------------------------------------
+__device__ __forceinline__ void clc_try_cancel(void* smem_answer, uint64_t* bar) {
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+                 ::"r"(smem_u32(smem_answer)), "r"(smem_u32(bar))
+                 : "memory");
+}
+// True when a block was taken over; x, y, z are then its index in the grid.
+__device__ __forceinline__ bool clc_read_answer(const void* smem_answer, int& x, int& y, int& z) {
+    uint32_t taken, cx, cy, cz;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b128 r;\n\t"
+        "ld.shared.b128 r, [%4];\n\t"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "mov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, %2, %3, _}, r;\n\t}"
+        : "=&r"(taken), "=&r"(cx), "=&r"(cy), "=&r"(cz)
+        : "r"(smem_u32(smem_answer))
+        : "memory");
+    x = (int)cx;
+    y = (int)cy;
+    z = (int)cz;
+    return taken != 0;
+}
+
+// ----------------------------------------------------------------------------
 // TMEM allocation (one warp, all 32 lanes; columns: power of two, 32..512)
 // ----------------------------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_result, uint32_t ncols) {

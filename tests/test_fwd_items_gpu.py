@@ -1,0 +1,76 @@
+"""GPU tests of the forward's work items: a thread block works through its own item and then takes over blocks that have
+not started (several per SM here), with rings and barrier phases running on; items of one key block, pairs whose second
+tile is missing or holds one row, the line between one and two query tiles per item, packed batches with items to pass
+over.  Parity per (sequence, KV head) against fp32 attention; tolerances are the common ones of the forward (bf16 P and
+O)."""
+import pytest
+import torch
+
+import util
+from hopper_jeni_b200 import ops
+from oracle import sdpa_ref
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(o, lse, q, k, v, scale, causal):  # [G, S, D], [G, S]; k, v [S, D]
+    torch.backends.cuda.matmul.allow_tf32 = False
+    z = torch.matmul(q.float(), k.float().t()) * scale
+    if causal:
+        z.masked_fill_(torch.ones_like(z[0], dtype=torch.bool).triu_(1), float("-inf"))
+    lse_ref, o_ref = torch.logsumexp(z, -1), torch.matmul(torch.softmax(z, -1), v.float())
+    m = sdpa_ref.metrics(o, o_ref)
+    assert m["finite"] and m["gate_ok"] and m["rel_rms"] <= util.REL_RMS_FWD, m
+    torch.testing.assert_close(lse, lse_ref, rtol=1e-3, atol=2e-3)
+
+
+BATCHED = [
+    # B, Hq, Hkv, S, D
+    (8, 24, 8, 300, 64),     # 384 items of three tiles (two + one) on 148 SMs
+    (8, 24, 8, 385, 128),    # the fourth tile holds one row
+    (16, 32, 4, 70, 64),     # 512 items of one key block
+    (16, 32, 4, 130, 128),   # one key block and two keys
+    (1, 4, 2, 4731, 64),     # 148 tiles: one tile per item
+    (1, 4, 2, 4737, 128),    # 152 tiles: two per item, the last one of a head holds one row
+    (5, 6, 2, 640, 40),      # 150 tiles, head dimension below the kernel's
+]
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("shape", BATCHED)
+def test_items_batched(gqa_lib, shape, causal):
+    B, Hq, Hkv, S, D = shape
+    G = Hq // Hkv
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    q, k, v = (torch.randn(B, h, S, D, generator=gen, device="cuda").bfloat16() for h in (Hq, Hkv, Hkv))
+    o, lse = torch.full_like(q, float("nan")), torch.full((B, Hq, S), float("nan"), device="cuda")
+    scale = util.default_scale(D)
+    ops.gqa_forward(q, k, v, causal=causal, scale=scale, out=o, lse=lse)
+    ops.check_status()
+    for b in range(B):
+        for g in range(Hkv):
+            h = slice(g * G, (g + 1) * G)
+            _check(o[b, h], lse[b, h], q[b, h], k[b, g], v[b, g], scale, causal)
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("D", [64, 128])
+def test_items_packed(gqa_lib, D, causal):
+    Hq, Hkv = 8, 2
+    G = Hq // Hkv
+    lens = [1, 0, 700, 128, 129, 0, 256, 33, 1500, 64, 257, 2, 511, 0, 90, 384] * 2
+    T = sum(lens)
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    q, k, v = (torch.randn(T, h, D, generator=gen, device="cuda").bfloat16() for h in (Hq, Hkv, Hkv))
+    cu = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device="cuda")
+    o, lse = torch.full_like(q, float("nan")), torch.full((Hq, T), float("nan"), device="cuda")
+    scale = util.default_scale(D)
+    ops.gqa_forward_varlen(q, k, v, cu, 2048, causal=causal, scale=scale, out=o, lse=lse)
+    ops.check_status()
+    start = 0
+    for n in lens:
+        r = slice(start, start + n)
+        start += n
+        for g in range(Hkv if n else 0):
+            h = slice(g * G, (g + 1) * G)
+            _check(o[r, h].transpose(0, 1), lse[h, r], q[r, h].transpose(0, 1), k[r, g], v[r, g], scale, causal)
