@@ -25,7 +25,7 @@
 //   warps 0-3    drain dQ tiles from TMEM into the fp32 accumulator
 //   warps 4-19   four elementwise warpgroups; each owns 32 query columns of the tile pair
 //   warp  20     TMA producer
-//   warps 21-23  UMMA issuers: [S^T, dP^T] | dV | [dK, dQ]
+//   warps 21-23  UMMA issuers: [S^T, dP^T] | dV | [dK, dQ] (dQ first at D = 128)
 // The five GEMMs wait on different producers, and one issuing warp sustains a 128x64x16 product
 // only every 57 cycles (78 when A comes from TMEM) against 32 cycles of tensor math, so they are
 // issued by three warps in parallel, each a warp-uniform loop with one elected lane; mbarriers
@@ -151,6 +151,11 @@ struct BwdCfg {
     // and dQ reuses the dP^T columns; the p_free / dq_empty barriers guard the reuse.
     static constexpr bool kPAliasesS = (D != 64);
     static constexpr bool kDqAliasesDp = (D != 64);
+    // dQ before dK where dQ sits in the dP^T columns: the loop dP^T -> dS^T -> dQ -> drain -> next dP^T then does not
+    // contain dK, which runs while the drain warps empty the columns.  B200, dK first -> dQ first: B4 Hq32 Hkv8 S8192 D128
+    // causal 5 499 -> 5 248 us, B8 Hq12 Hkv4 S4096 D128 2 061 -> 1 984 us, B2 Hq24 S4096 D128 causal with ordered dQ
+    // 865 -> 842 us.  (At D = 64 dQ has columns of its own and the next dP^T waits for dK instead.)
+    static constexpr bool kDqFirst = kDqAliasesDp;
     // D = 64: dS^T is also stored as bf16 over the first half of each warpgroup's dP^T columns, so that dK reads
     // its A operand from TMEM instead of shared memory (shared-memory bandwidth is what bounds this kernel).
     static constexpr bool kDsInTmem = (D == 64);
@@ -229,7 +234,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     uint64_t* kv_full = bars + 0;    // TMA: K and V tiles
     uint64_t* p_ready = bars + 1;    // elementwise -> issuers: P^T(it) stored, S^T(it) consumed
     uint64_t* ds_ready = bars + 2;   // elementwise -> issuers: dS^T(it) stored, dP^T(it) consumed
-    uint64_t* ds_free = bars + 3;    // after dQ(it) (covers dK(it), same thread): dS^T(it) consumed, dQ(it) complete
+    uint64_t* dq_full = bars + 3;    // after dQ(it): -> drain warps
     uint64_t* dq_empty = bars + 4;   // drain warps -> issuers: dQ columns free
     uint64_t* acc_full = bars + 5;   // issuers dV + dK after the last products of a work item -> epilogue
     uint64_t* acc_empty = bars + 6;  // elementwise -> issuers dV + dK: the accumulators of the item have been read
@@ -237,6 +242,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     uint64_t* s_full = bars + 8;                     // [kQStages] after S^T(it): -> elementwise
     uint64_t* dk_done = s_full + Cfg::kQStages;      // [kQStages] after dK(it): Q stage free (S^T(it) finished long before),
                                                      //            and the dS^T copy in the dP^T columns has been read
+                                                     //            (covers dQ(it) where that is issued first, same thread)
     uint64_t* q_full = dk_done + Cfg::kQStages;      // [kQStages] TMA: Q tile + -LSE/scale columns
     uint64_t* dp_full = q_full + Cfg::kQStages;      // [kDOStages] after dP^T(it): -> elementwise; dO stage read by dP^T
     uint64_t* p_free = dp_full + Cfg::kDOStages;     // [kDOStages] after dV(it): P^T(it) consumed; dO stage read by dV
@@ -346,7 +352,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
         mbar_init(kv_full, 1);
         mbar_init(p_ready, Cfg::kEwThreads);
         mbar_init(ds_ready, Cfg::kEwThreads);
-        mbar_init(ds_free, 1);
+        mbar_init(dq_full, 1);
         mbar_init(dq_empty, 128);
         mbar_init(acc_full, 2);
         mbar_init(acc_empty, Cfg::kEwThreads);
@@ -561,34 +567,37 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                 tc_fence_after_sync();
                 GQA_TRACE(4, gi, 0);
                 const uint32_t b0 = q_addr + qs * Cfg::kTileBytes;
-                const uint32_t ds_buf = ds_addr;
+                auto issue_dk = [&]() {
 #pragma unroll
-                for (int kk = 0; kk < 8; ++kk) {
-                    if constexpr (Cfg::kDsInTmem)  // A = bf16 dS^T in the dP^T columns: query columns [16kk, 16kk+16)
-                        umma_ts_pred(leader, tmem + Cfg::kColDK, tmem + Cfg::kColDP + (kk / Cfg::kHalves) * Cfg::kCols + (kk % Cfg::kHalves) * 8,
-                                     make_sdesc_sw128(b0 + kk * 2048, kPanel, 1024), idesc, (it > 0 || kk > 0));
-                    else
-                        umma_ss_pred(leader, tmem + Cfg::kColDK,
-                                     make_sdesc_sw128(ds_buf + (kk >> 2) * kPanel + (kk & 3) * 32, 16, 1024),
-                                     make_sdesc_sw128(b0 + kk * 2048, kPanel, 1024), idesc, (it > 0 || kk > 0));
-                }
-                umma_commit_pred(leader, &dk_done[qs]);
-                GQA_TRACE(4, gi, 1);
-                if constexpr (!kWithDQ) {
-                    umma_commit_pred(leader, ds_free);  // dK(it) was the last reader of dS^T(it)
-                } else {  // dQ(it) = dS K  (A = dS^T read MN-major, B = K read MN-major)
-                    if (gi > 0) ok = mbar_wait(dq_empty, (gi - 1) & 1, ctx, 36);
-                    if (!ok) break;
+                    for (int kk = 0; kk < 8; ++kk) {
+                        if constexpr (Cfg::kDsInTmem)  // A = bf16 dS^T in the dP^T columns: query columns [16kk, 16kk+16)
+                            umma_ts_pred(leader, tmem + Cfg::kColDK, tmem + Cfg::kColDP + (kk / Cfg::kHalves) * Cfg::kCols + (kk % Cfg::kHalves) * 8,
+                                         make_sdesc_sw128(b0 + kk * 2048, kPanel, 1024), idesc, (it > 0 || kk > 0));
+                        else
+                            umma_ss_pred(leader, tmem + Cfg::kColDK,
+                                         make_sdesc_sw128(ds_addr + (kk >> 2) * kPanel + (kk & 3) * 32, 16, 1024),
+                                         make_sdesc_sw128(b0 + kk * 2048, kPanel, 1024), idesc, (it > 0 || kk > 0));
+                    }
+                    umma_commit_pred(leader, &dk_done[qs]);
+                    GQA_TRACE(4, gi, 1);
+                };
+                auto issue_dq = [&]() -> bool {  // A = dS^T read MN-major, B = K read MN-major
+                    if (gi > 0 && !mbar_wait(dq_empty, (gi - 1) & 1, ctx, 36)) return false;
                     tc_fence_after_sync();
                     GQA_TRACE(4, gi, 2);
                     const uint32_t idesc_dq = make_idesc_bf16(128, D, true, true);
 #pragma unroll
                     for (int kk = 0; kk < 8; ++kk)
-                        umma_ss_pred(leader, tmem + Cfg::kColDQ, make_sdesc_sw128(ds_buf + kk * 2048, kPanel, 1024),
+                        umma_ss_pred(leader, tmem + Cfg::kColDQ, make_sdesc_sw128(ds_addr + kk * 2048, kPanel, 1024),
                                      make_sdesc_sw128(k_addr + kk * 2048, kPanel, 1024), idesc_dq, kk > 0);
-                    umma_commit_pred(leader, ds_free);
+                    umma_commit_pred(leader, dq_full);
                     GQA_TRACE(4, gi, 3);
-                }
+                    return true;
+                };
+                if constexpr (kWithDQ && Cfg::kDqFirst) ok = issue_dq();
+                if (!ok) break;
+                issue_dk();
+                if constexpr (kWithDQ && !Cfg::kDqFirst) ok = issue_dq();
             }
             if (ok) {
                 umma_commit_pred(leader, acc_full);
@@ -672,7 +681,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
             bool turn_mine = !kDet;  // becomes true once this warp may reduce into the slice
             // first look at the counter now: its round trip to L2 hides behind the TMEM loads and the staging
             const unsigned int early = (kDet && lane == 0) ? ld_acquire_gpu(turn) : 0xffffffffu;
-            if (!mbar_wait(ds_free, gi & 1, ctx, 40)) { going = false; break; }  // dQ(it) complete
+            if (!mbar_wait(dq_full, gi & 1, ctx, 40)) { going = false; break; }  // dQ(it) complete
             tc_fence_after_sync();
             GQA_TRACE(2, gi, 0);
             constexpr int kRounds = D / (32 * Cfg::kDqBoxes);
@@ -978,7 +987,10 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                 if (++qi == n_qt) qi = 0;
                 if (!ok) break;
                 ok = mbar_wait(&dp_full[gi % Cfg::kDOStages], (gi / Cfg::kDOStages) & 1, ctx, 53);
-                if (ok && gi > 0) ok = mbar_wait(ds_free, (gi - 1) & 1, ctx, 54);  // dK and dQ of the iteration before have read its dS^T
+                if (ok && gi > 0) {  // dK and dQ of the iteration before have read its dS^T: the later of the two has completed
+                    if constexpr (kWithDQ && !Cfg::kDqFirst) ok = mbar_wait(dq_full, (gi - 1) & 1, ctx, 54);
+                    else ok = mbar_wait(&dk_done[(gi - 1) % Cfg::kQStages], ((gi - 1) / Cfg::kQStages) & 1, ctx, 54);
+                }
                 if (!ok) break;
                 tc_fence_after_sync();
                 if (trace_me) GQA_TRACE(0, gi, 0);
