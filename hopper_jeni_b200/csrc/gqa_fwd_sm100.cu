@@ -78,7 +78,10 @@ struct FwdParams {
     float scale_log2;  // scale * log2(e)
 };
 
-template <int D>
+// kMore: the launch has more items than SMs, so blocks ask for further ones; without it the kernel is the plain
+// one-item-per-block form (every running count below is a constant 0 there): a launch of the kMore form that has nothing to
+// hand out is 1.5 us slower at B1 Hq4 S128 D64 (8.2 against 6.7 us) and 3 % at B2 Hq12 S1000 D128.
+template <int D, bool kMore>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                      const __grid_constant__ CUtensorMap mapV, const FwdParams p) {
@@ -135,7 +138,7 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     // Packed variable-length batch: the sequence is a row range [y0, y0 + len) of the one [T, H*D] matrix; rows past
     // its end belong to the next sequence (or read as zeros past T): as keys they are masked like keys beyond S,
     // as queries they are computed and not stored.  The grid covers max_seqlen: an item beyond its sequence has
-    // n_tiles = 0 and is passed over by the producer.
+    // n_tiles = 0 and no key blocks; a block's own may be such a one, further ones are passed over by the producer.
     auto decode = [&](int x, int y, int z) -> Item {
         Item w;
         const int idx = p.causal ? (p.n_groups - 1 - x) : x;  // heavy causal tiles first
@@ -151,18 +154,25 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
         }
         w.n_tiles = w.q0 >= w.len ? 0 : (p.tiles == 2 && w.q0 + kTile < w.len) ? 2 : 1;
         const int n_blocks_all = (w.len + kTile - 1) / kTile;  // the last block may be partial: keys at and beyond len are masked
-        w.n_blk0 = p.causal ? (w.q0 / kTile + 1) : n_blocks_all;
+        w.n_blk0 = (w.n_tiles == 0) ? 0 : p.causal ? (w.q0 / kTile + 1) : n_blocks_all;
         w.n_blk1 = (w.n_tiles == 2) ? (p.causal ? (w.q0 / kTile + 2) : n_blocks_all) : 0;
         w.n_max = max(w.n_blk0, w.n_blk1);
         return w;
     };
-    // The j-th item of this block, published by the producer: false = no more (or give up).
+    // The j-th item of this block: its own, which every role knows, then the ones that the producer publishes.
+    // False = no more (or give up).
     auto fetch_item = [&](int j, Item& w) -> bool {
-        const int sl = j % kItemSlots;
-        if (!mbar_wait(&item_full[sl], (j / kItemSlots) & 1, ctx, 14)) return false;
-        const int x = item_slot[sl * 4 + 0], y = item_slot[sl * 4 + 1], z = item_slot[sl * 4 + 2];
-        mbar_arrive(&item_empty[sl]);
-        if (x < 0) return false;
+        int x = blockIdx.x, y = blockIdx.y, z = blockIdx.z;
+        if (j > 0) {
+            if constexpr (!kMore) return false;
+            const int sl = (j - 1) % kItemSlots;
+            if (!mbar_wait(&item_full[sl], ((j - 1) / kItemSlots) & 1, ctx, 14)) return false;
+            x = item_slot[sl * 4 + 0];
+            y = item_slot[sl * 4 + 1];
+            z = item_slot[sl * 4 + 2];
+            mbar_arrive(&item_empty[sl]);
+            if (x < 0) return false;
+        }
         w = decode(x, y, z);
         return true;
     };
@@ -234,22 +244,23 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                 }
             };
             bool ok = true;
-            if (p.cu && decode(x, y, z).n_tiles == 0) ok = claim();
             uint32_t kb = 0;             // key blocks loaded so far, over all items
             int n_q[2] = {0, 0};         // loads of the two Q tiles so far
             for (int j = 0; ok; ++j) {
-                const int sl = j % kItemSlots;
-                if (j >= kItemSlots && !mbar_wait(&item_empty[sl], (j / kItemSlots - 1) & 1, ctx, 13)) break;
-                // a block of this launch that gave up has left a non-zero status word: stop taking items
-                if (j > 0 && *reinterpret_cast<volatile unsigned int*>(p.status) != 0u) {
-                    *abort_flag = 98u;
-                    break;
+                if (j > 0) {
+                    const int sl = (j - 1) % kItemSlots, use = (j - 1) / kItemSlots;
+                    if (use > 0 && !mbar_wait(&item_empty[sl], (use - 1) & 1, ctx, 13)) break;
+                    // a block of this launch that gave up has left a non-zero status word: stop taking items
+                    if (*reinterpret_cast<volatile unsigned int*>(p.status) != 0u) {
+                        *abort_flag = 98u;
+                        break;
+                    }
+                    item_slot[sl * 4 + 0] = x;
+                    item_slot[sl * 4 + 1] = y;
+                    item_slot[sl * 4 + 2] = z;
+                    mbar_arrive(&item_full[sl]);
+                    if (x < 0) break;
                 }
-                item_slot[sl * 4 + 0] = x;
-                item_slot[sl * 4 + 1] = y;
-                item_slot[sl * 4 + 2] = z;
-                mbar_arrive(&item_full[sl]);
-                if (x < 0) break;
                 const Item w = decode(x, y, z);
                 const int hkv = w.hq / (p.Hq / p.Hkv);
                 // Tensor-map coordinates (x = column, y = position in the sequence, z = matrix).  [B,H,S,D] is B*H matrices
@@ -275,6 +286,7 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                     for (int pn = 0; pn < Cfg::kPanels; ++pn)
                         tma_load_3d(sV + st * Cfg::kTileBytes + pn * kPanel, &mapV, &v_full[st], kv_x + pn * 64, w.y0 + n * kTile, kv_z);
                 }
+                if constexpr (!kMore) break;
                 if (ok) ok = claim();
             }
         }
@@ -312,7 +324,7 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                     }
                     umma_commit_pred(leader, &s_full[t * 2 + h]);
                     if (h == 1) umma_commit_pred(leader, &k_empty[st]);
-                    if (h == 1 && n + 1 == n_blk) umma_commit_pred(leader, &q_empty[t]);
+                    if (kMore && h == 1 && n + 1 == n_blk) umma_commit_pred(leader, &q_empty[t]);
                     if (t == 0) GQA_FTRACE(1, 2 * n + h, 0);
                     return true;
                 };
@@ -352,6 +364,7 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                 if (ok) ok = mbar_wait(&v_full[st], par, ctx, 27);
                 if (ok && leader) mbar_arrive(&v_empty[st]);
             }
+            if constexpr (!kMore) break;
             kb += n_max;
             cb += n_blk;
         }
@@ -364,7 +377,10 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
         Item w;
         for (int it = 0; ok && fetch_item(it, w); ++it) {
             const int n_blk = t ? w.n_blk1 : w.n_blk0;
-            if (n_blk == 0) continue;
+            if (n_blk == 0) {
+                if constexpr (kMore) continue;
+                else break;
+            }
             const int q0 = w.q0, len = w.len, hq = w.hq, b = w.b, y0 = w.y0;
             const int q_row0 = (b * p.Hq + hq) * p.S + y0 + q0;   // row in [B,Hq,S] order (LSE)
             const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
@@ -518,6 +534,7 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                 tc_fence_before_sync();
                 mbar_arrive(&o_empty[t]);
             }
+            if constexpr (!kMore) break;
             cb += n_blk;
             ++n_done;
         }
@@ -547,8 +564,6 @@ int launch_fwd_t(const void* Q, const void* K, const void* V, void* O, float* LS
     if (rc) return rc;
     rc = make_tile3_tmap(&mv, V, kc, S, nkv, S * kc, kTile);
     if (rc) return rc;
-    GQA_CUDA_TRY(cudaFuncSetAttribute(gqa_fwd_sm100_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      Cfg::kSmemTotal));
     FwdParams p;
     p.O = static_cast<__nv_bfloat16*>(O);
     p.LSE = LSE;
@@ -568,7 +583,9 @@ int launch_fwd_t(const void* Q, const void* K, const void* V, void* O, float* LS
     p.n_groups = (n_tiles + p.tiles - 1) / p.tiles;
     p.scale_log2 = s.scale * kLog2e;
     dim3 grid(p.n_groups, s.Hq, n_seqs);
-    gqa_fwd_sm100_kernel<D><<<grid, kFwdThreads, Cfg::kSmemTotal, stream>>>(mq, mk, mv, p);
+    auto kernel = (long long)p.n_groups * s.Hq * n_seqs > sm_count() ? gqa_fwd_sm100_kernel<D, true> : gqa_fwd_sm100_kernel<D, false>;
+    GQA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemTotal));
+    kernel<<<grid, kFwdThreads, Cfg::kSmemTotal, stream>>>(mq, mk, mv, p);
     count_launch();
     GQA_CUDA_TRY(cudaGetLastError());
     return GQA_OK;
