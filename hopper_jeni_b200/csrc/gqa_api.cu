@@ -171,16 +171,11 @@ int run_bwd(const void* Q, const void* K, const void* V, const void* O, const vo
     // form except at one shape, so the separate pass is taken only when asked for.
     const bool dq_separate = (flags & GQA_BWD_DQ_SEPARATE) != 0;
     unsigned int* dq_turn = nullptr;
-    if ((flags & GQA_BWD_DETERMINISTIC) && !dq_separate) {
-        dq_turn = reinterpret_cast<unsigned int*>(w + ws.dq_turn_off);
-        GQA_CUDA_TRY(cudaMemsetAsync(dq_turn, 0, ws.dq_turn_bytes, stream));
-    }
-
-    GQA_CUDA_TRY(cudaMemsetAsync(status, 0, 256, stream));
+    if ((flags & GQA_BWD_DETERMINISTIC) && !dq_separate) dq_turn = reinterpret_cast<unsigned int*>(w + ws.dq_turn_off);
     if (ev) GQA_CUDA_TRY(cudaEventRecord(ev[0], stream));
     rc = gqa::launch_bwd_preprocess(O, dO, LSE, 1.0f / scale, dq_separate ? delta_f32 : nullptr, lse_cols, delta_cols,
                                     dq_separate ? nullptr : dq_accum, s.q_rows(), D, stream, s.bshd ? S : 0,
-                                    s.bshd ? Hq : 0);
+                                    s.bshd ? Hq : 0, status, dq_turn, dq_turn ? ws.dq_turn_bytes / sizeof(unsigned int) : 0);
     if (rc) return rc;
     if (ev) GQA_CUDA_TRY(cudaEventRecord(ev[1], stream));
     float* partial = parts > 1 ? reinterpret_cast<float*>(w + ws.partial_off) : nullptr;

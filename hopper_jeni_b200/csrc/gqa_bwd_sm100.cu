@@ -212,6 +212,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     using Cfg = BwdCfg<D>;
     extern __shared__ __align__(1024) uint8_t smem[];
     if ((smem_u32(smem) & 1023u) != 0) {  // swizzled panels need 1024-byte alignment; report instead of computing garbage
+        pdl_wait();
         if (threadIdx.x == 0) atomicCAS(p.status, 0u, 0x80000000u | (99u << 20));
         return;
     }
@@ -345,10 +346,8 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     auto q_z_of = [&](const WorkItem& w, int it) { return p.bshd ? w.b : w.b * p.Hq + head_of(w, it); };
     auto ws_z_of = [&](const WorkItem& w, int it) { return w.b * p.Hq + head_of(w, it); };
 
+    pdl_launch_dependents();
     if (tid == 0) {
-        // a thread block of this launch that has already given up leaves a non-zero status word: the blocks that
-        // start after it skip their work (see below), so a wedged launch drains in one wave
-        *abort_flag = (*reinterpret_cast<volatile unsigned int*>(p.status) != 0u) ? 98u : 0u;
         mbar_init(kv_full, 1);
         mbar_init(p_ready, Cfg::kEwThreads);
         mbar_init(ds_ready, Cfg::kEwThreads);
@@ -379,6 +378,11 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
         *reinterpret_cast<uint4*>(sZero + tid * 16) = make_uint4(0u, 0u, 0u, 0u);
         fence_proxy_async_smem();
     }
+    // Everything above overlaps the end of the preprocess kernel, whose output (workspace) is first used from here on.
+    pdl_wait();
+    // a thread block of this launch that has already given up leaves a non-zero status word: the blocks that
+    // start after it skip their work (see below), so a wedged launch drains in one wave
+    if (tid == 0) *abort_flag = (*reinterpret_cast<volatile unsigned int*>(p.status) != 0u) ? 98u : 0u;
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -1110,9 +1114,8 @@ int launch_bwd_t(const void* Q, const void* K, const void* V, const void* dO, co
     // persistent, one block per SM (shared memory and TMEM allow no second), except in the deterministic mode (see the
     // work-item comment in the kernel)
     const unsigned grid = (unsigned)(dq_turn ? p.n_items : std::min(p.n_items, sm_count()));
-    kernel<<<grid, Cfg::kThreads, Cfg::kSmemTotal, stream>>>(mq, mk, mv, mdo, mdq, mlse, mdlt, p);
+    GQA_CUDA_TRY(launch_after(kernel, dim3(grid), Cfg::kThreads, Cfg::kSmemTotal, stream, mq, mk, mv, mdo, mdq, mlse, mdlt, p));
     count_launch();
-    GQA_CUDA_TRY(cudaGetLastError());
     return GQA_OK;
 }
 

@@ -41,6 +41,23 @@ int make_tile3_tmap(CUtensorMap* out, const void* base, uint64_t cols, uint64_t 
 int make_f32box3_tmap(CUtensorMap* out, const void* base, uint64_t cols, uint64_t S, uint64_t n_outer, uint32_t box_rows);
 int make_col8_3_tmap(CUtensorMap* out, const void* base, uint64_t S, uint64_t n_outer, uint32_t box_rows);
 
+// Launch whose blocks may start before the kernel in front of it in the stream has ended: the kernel must call pdl_wait()
+// (sm100_ptx.cuh) before it touches global memory.
+template <class... P, class... A>
+cudaError_t launch_after(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, A&&... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // SMs of the current device (1 when it cannot be asked).
 int sm_count();
 

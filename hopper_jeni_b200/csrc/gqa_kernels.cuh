@@ -54,10 +54,12 @@ struct BwdWorkspace {
 // Stage 1 of the backward: Delta = rowsum(dO*O); with `delta` it is stored as fp32, with the column arrays
 // the bf16 splits of -LSE*inv_scale and -Delta are stored (16 bytes per row each) and, if given, the dQ
 // accumulator is zeroed.
+// `status` (the 256 bytes in front of the workspace) and the `n_turns` words at `turns` are zeroed as well.
 // `S_bshd` / `H_bshd`: 0 when O, dO are in [B,H,S,D] order, else S and Hq of the [B,S,H,D] layout they are in.
 int launch_bwd_preprocess(const void* O, const void* dO, const float* lse, float inv_scale, float* delta,
                           void* lse_cols, void* delta_cols, float* dq_accum, size_t rows, int D, cudaStream_t stream,
-                          int S_bshd = 0, int H_bshd = 0);
+                          int S_bshd = 0, int H_bshd = 0, unsigned int* status = nullptr, unsigned int* turns = nullptr,
+                          size_t n_turns = 0);
 // Stage 3 of the backward: dQ = bf16(scale * dq_accum) (dQ in [B,S,H,D] order when S_bshd / H_bshd are given).
 // `rows` rows of Dp fp32 accumulator columns -> rows of D bf16 columns.
 int launch_dq_finalise(const float* dq_accum, void* dQ, size_t rows, float scale, cudaStream_t stream,

@@ -12,6 +12,7 @@
 
 #include "gqa_common.cuh"
 #include "gqa_kernels.cuh"
+#include "sm100_ptx.cuh"
 
 namespace gqa {
 
@@ -27,6 +28,9 @@ __device__ __forceinline__ uint2 split3_bf16(float x) {
                       (uint32_t)__bfloat16_as_ushort(lo));
 }
 
+constexpr int kStatusWords = 64;  // the status word and the work counter behind it: 256 bytes
+
+// (The words that the backward needs zeroed ride along: as memset nodes in front they were a launch each.)
 // One group of D/8 lanes per row; each lane owns 8 consecutive elements (one 16-byte load
 // from O and one from dO).  A warp covers 256/D rows per step.  D is the padded head dimension (64 or 128, the
 // width of an accumulator row); O and dO rows hold `d_real` <= D columns.
@@ -35,7 +39,10 @@ __global__ void __launch_bounds__(256)
 bwd_preprocess_kernel(const uint4* __restrict__ O, const uint4* __restrict__ dO, const float* __restrict__ lse,
                       float inv_scale, float* __restrict__ delta, uint4* __restrict__ lse_cols,
                       uint4* __restrict__ delta_cols, float4* __restrict__ dq_accum, size_t rows, int S_bshd, int H_bshd,
-                      int d_real) {
+                      int d_real, unsigned int* __restrict__ status, unsigned int* __restrict__ turns, size_t n_turns) {
+    sm100::pdl_launch_dependents();
+    if (status && blockIdx.x == 0 && threadIdx.x < kStatusWords) status[threadIdx.x] = 0u;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_turns; i += (size_t)gridDim.x * blockDim.x) turns[i] = 0u;
     constexpr int kLanesPerRow = D / 8;
     const int real8 = d_real / 8;  // 16-byte groups per O / dO row
     constexpr int kRowsPerWarp = 32 / kLanesPerRow;
@@ -84,8 +91,8 @@ bwd_preprocess_kernel(const uint4* __restrict__ O, const uint4* __restrict__ dO,
 // n8 groups of eight output elements; per8 = D / 8 groups per dQ row, acc8 = groups per accumulator row (the padded
 // head dimension / 8).  The accumulator is in [B,H,S] row order, dQ may be stored [B,S,H,D] (S_bshd, H_bshd non-zero).
 __global__ void __launch_bounds__(256)
-dq_finalise_kernel(const float4* __restrict__ acc, uint4* __restrict__ dq, size_t n8, float scale, int per8, int acc8,
-                   int S_bshd, int H_bshd) {
+dq_finalise_kernel(const float4* acc, uint4* dq, size_t n8, float scale, int per8, int acc8, int S_bshd, int H_bshd) {
+    sm100::pdl_wait();  // (no __restrict__: a load declared read-only for the kernel's life could be moved above this)
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (size_t)gridDim.x * blockDim.x) {
         const size_t src = (i / per8) * acc8 + i % per8;
         const float4 a = acc[2 * src], b = acc[2 * src + 1];
@@ -147,7 +154,7 @@ int grid_for(size_t work_items, int per_block) {
 
 int launch_bwd_preprocess(const void* O, const void* dO, const float* lse, float inv_scale, float* delta,
                           void* lse_cols, void* delta_cols, float* dq_accum, size_t rows, int D, cudaStream_t stream,
-                          int S_bshd, int H_bshd) {
+                          int S_bshd, int H_bshd, unsigned int* status, unsigned int* turns, size_t n_turns) {
     const int Dp = D <= 64 ? 64 : 128;
     const int rows_per_block = (256 / 32) * (256 / Dp);
     const int grid = grid_for(rows, rows_per_block);
@@ -155,12 +162,14 @@ int launch_bwd_preprocess(const void* O, const void* dO, const float* lse, float
         bwd_preprocess_kernel<64><<<grid, 256, 0, stream>>>(static_cast<const uint4*>(O), static_cast<const uint4*>(dO),
                                                             lse, inv_scale, delta, static_cast<uint4*>(lse_cols),
                                                             static_cast<uint4*>(delta_cols),
-                                                            reinterpret_cast<float4*>(dq_accum), rows, S_bshd, H_bshd, D);
+                                                            reinterpret_cast<float4*>(dq_accum), rows, S_bshd, H_bshd, D, status,
+                                                            turns, n_turns);
     else
         bwd_preprocess_kernel<128><<<grid, 256, 0, stream>>>(static_cast<const uint4*>(O), static_cast<const uint4*>(dO),
                                                              lse, inv_scale, delta, static_cast<uint4*>(lse_cols),
                                                             static_cast<uint4*>(delta_cols),
-                                                            reinterpret_cast<float4*>(dq_accum), rows, S_bshd, H_bshd, D);
+                                                            reinterpret_cast<float4*>(dq_accum), rows, S_bshd, H_bshd, D, status,
+                                                            turns, n_turns);
     count_launch();
     GQA_CUDA_TRY(cudaGetLastError());
     return GQA_OK;
@@ -170,10 +179,9 @@ int launch_dq_finalise(const float* dq_accum, void* dQ, size_t rows, float scale
                        int S_bshd, int H_bshd) {
     const size_t n8 = rows * (size_t)(D / 8);
     const int grid = grid_for(n8, 256);
-    dq_finalise_kernel<<<grid, 256, 0, stream>>>(reinterpret_cast<const float4*>(dq_accum), static_cast<uint4*>(dQ), n8,
-                                                 scale, D / 8, (D <= 64 ? 64 : 128) / 8, S_bshd, H_bshd);
+    GQA_CUDA_TRY(launch_after(dq_finalise_kernel, dim3(grid), 256, 0, stream, reinterpret_cast<const float4*>(dq_accum),
+                              static_cast<uint4*>(dQ), n8, scale, D / 8, (D <= 64 ? 64 : 128) / 8, S_bshd, H_bshd));
     count_launch();
-    GQA_CUDA_TRY(cudaGetLastError());
     return GQA_OK;
 }
 

@@ -162,6 +162,14 @@ __device__ __forceinline__ void st_release_gpu(unsigned int* p, unsigned int v) 
 }
 
 // ----------------------------------------------------------------------------
+// Programmatic dependent launch.  A kernel launched with launch_after() (gqa_common.cuh) may start while the one before it
+// in the stream still runs, once every block of that one has called pdl_launch_dependents() or ended; pdl_wait() returns when
+// that one has completed and its writes are visible.  Nothing it wrote, and nothing it may still read, is touched before.
+// ----------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// ----------------------------------------------------------------------------
 // Cluster launch control: a running thread block takes over a block of its own launch that has not started yet.
 // The request is asynchronous; its 16-byte answer lands in shared memory (16-byte aligned) and completes 16 bytes of
 // transactions on the mbarrier.  After an answer "nothing left" no further request may be made.
