@@ -294,7 +294,7 @@ extern "C" int gqa_bwd_static_scratch(const void* Q, const void* K, const void* 
     void* scratch = nullptr;
     rc = static_scratch_address(&scratch);
     if (rc) return rc;
-    // run_bwd clears the status word and the preprocess stage zeroes the dQ accumulator, so nothing
+    // the preprocess stage clears the status word and zeroes the dQ accumulator, so nothing
     // left in the array by an earlier call is read.
     return run_bwd(Q, K, V, O, dO, LSE, dQ, dK, dV, B, Hq, Hkv, S, D, causal, scale, scratch, need,
                    reinterpret_cast<cudaStream_t>(stream), nullptr);
