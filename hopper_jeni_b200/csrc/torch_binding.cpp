@@ -73,8 +73,14 @@ int as_int(int64_t v) {
     return static_cast<int>(v);
 }
 
+// K against Q (V, dK and dV are compared with K, everything else with Q): nothing of a call is on another device.
+void require_same_device(const Tensor& q, const Tensor& k) {
+    TORCH_CHECK_VALUE(k.device() == q.device(), "K is on ", k.device(), ", expected ", q.device());
+}
+
 Dims dims(const Tensor& q, const Tensor& k, bool bshd) {
     TORCH_CHECK_VALUE(q.dim() == 4 && k.dim() == 4, "Q and K/V must be 4-dimensional");
+    require_same_device(q, k);
     const int seq = bshd ? 1 : 2, head = bshd ? 2 : 1;
     TORCH_CHECK_VALUE(k.size(0) == q.size(0) && k.size(seq) == q.size(seq) && k.size(3) == q.size(3), "K/V shape ",
                       k.sizes(), " does not match Q ", q.sizes());
@@ -83,6 +89,7 @@ Dims dims(const Tensor& q, const Tensor& k, bool bshd) {
 
 Dims packed_dims(const Tensor& q, const Tensor& k, const Tensor& cu) {
     TORCH_CHECK_VALUE(q.dim() == 3 && k.dim() == 3, "packed batches are [total_tokens, H, D]");
+    require_same_device(q, k);
     TORCH_CHECK_VALUE(k.size(0) == q.size(0) && k.size(2) == q.size(2), "K ", k.sizes(), " does not match Q ", q.sizes());
     TORCH_CHECK_VALUE(cu.scalar_type() == at::kInt && cu.dim() == 1 && cu.numel() >= 2 && cu.is_cuda() &&
                           cu.device() == q.device() && cu.is_contiguous(),
