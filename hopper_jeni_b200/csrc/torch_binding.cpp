@@ -101,12 +101,36 @@ float scale_or_default(double scale, int D) {  // NaN: not given
     return static_cast<float>(std::isnan(scale) ? 1.0 / std::sqrt(static_cast<double>(D)) : scale);
 }
 
-gqa_stream_t stream_of(const Tensor& q, const std::optional<uintptr_t>& given) {
-    if (given) return reinterpret_cast<gqa_stream_t>(*given);
-    return c10::cuda::getCurrentCUDAStream(q.get_device()).stream();
-}
+// The device and the stream of one call, current for as long as this lives.  A stream that was given and is not the
+// caller's current one owns what the call allocates: torch's allocator orders the reuse of a block by its stream, so a
+// workspace taken from the current stream's pool could be handed out again, and an output could be memory that the
+// current stream still uses, while the kernels run on the given one.
+class CallStream {
+public:
+    CallStream(const Tensor& q, const std::optional<uintptr_t>& given)
+        : device_(q.device()), caller_(c10::cuda::getCurrentCUDAStream(q.get_device())), handle_(caller_.stream()) {
+        if (!given || reinterpret_cast<cudaStream_t>(*given) == caller_.stream()) return;
+        const auto run = c10::cuda::getStreamFromExternal(reinterpret_cast<cudaStream_t>(*given), q.get_device());
+        handle_ = run.stream();
+        given_.emplace(run);
+    }
+    gqa_stream_t handle() const { return handle_; }
+    // A tensor that goes back to the caller: its block is not reused before the caller's stream is done with it, either.
+    Tensor returned(Tensor t) const {
+        if (given_) t.record_stream(caller_.unwrap());
+        return t;
+    }
+    Tensor empty_like(const Tensor& t) const { return returned(at::empty_like(t)); }
+    Tensor empty_f32(const Tensor& like, at::IntArrayRef shape) const {
+        return returned(at::empty(shape, like.options().dtype(at::kFloat)));
+    }
 
-Tensor empty_f32(const Tensor& like, at::IntArrayRef shape) { return at::empty(shape, like.options().dtype(at::kFloat)); }
+private:
+    const c10::cuda::CUDAGuard device_;
+    const c10::cuda::CUDAStream caller_;
+    gqa_stream_t handle_;
+    std::optional<c10::cuda::CUDAStreamGuard> given_;
+};
 
 struct CallArgs {
     bool causal = false, bshd = false;
@@ -127,15 +151,15 @@ std::tuple<Tensor, Tensor> forward(const Tensor& q, const Tensor& k, const Tenso
     check_qkv(q, k, v);
     const Dims d = dims(q, k, a.bshd);
     require_like(v, "V", k);
-    const c10::cuda::CUDAGuard guard(q.device());
     const int64_t lse_shape[3] = {d.B, d.Hq, d.S};
     if (out) require_like(*out, "O", q);
-    else out = at::empty_like(q);
     if (lse) require_like(*lse, "LSE", q, lse_shape, at::kFloat);
-    else lse = empty_f32(q, lse_shape);
+    const CallStream stream(q, a.stream);
+    if (!out) out = stream.empty_like(q);
+    if (!lse) lse = stream.empty_f32(q, lse_shape);
     check_status("gqa_fwd_ex", api.fwd_ex(q.data_ptr(), k.data_ptr(), v.data_ptr(), out->data_ptr(),
                                           static_cast<float*>(lse->data_ptr()), d.B, d.Hq, d.Hkv, d.S, d.D, a.causal,
-                                          scale_or_default(a.scale, d.D), stream_of(q, a.stream),
+                                          scale_or_default(a.scale, d.D), stream.handle(),
                                           a.bshd ? GQA_LAYOUT_BSHD : 0u));
     return {std::move(*out), std::move(*lse)};
 }
@@ -146,17 +170,17 @@ std::tuple<Tensor, Tensor> forward_varlen(const Tensor& q, const Tensor& k, cons
     check_qkv(q, k, v);
     const Dims d = packed_dims(q, k, cu);
     require_like(v, "V", k);
-    const c10::cuda::CUDAGuard guard(q.device());
     const int64_t lse_shape[2] = {d.Hq, d.S};
     if (out) require_like(*out, "O", q);
-    else out = at::empty_like(q);
     if (lse) require_like(*lse, "LSE", q, lse_shape, at::kFloat);
-    else lse = empty_f32(q, lse_shape);
+    const CallStream stream(q, a.stream);
+    if (!out) out = stream.empty_like(q);
+    if (!lse) lse = stream.empty_f32(q, lse_shape);
     check_status("gqa_fwd_varlen",
                  api.fwd_varlen(q.data_ptr(), k.data_ptr(), v.data_ptr(), out->data_ptr(),
                                 static_cast<float*>(lse->data_ptr()), static_cast<const int*>(cu.data_ptr()),
                                 as_int(cu.numel()) - 1, d.S, as_int(max_seqlen), d.Hq, d.Hkv, d.D, a.causal,
-                                scale_or_default(a.scale, d.D), stream_of(q, a.stream)));
+                                scale_or_default(a.scale, d.D), stream.handle()));
     return {std::move(*out), std::move(*lse)};
 }
 
@@ -175,21 +199,24 @@ struct BwdTensors {
         require(dout, "dO", at::kBFloat16);
         require(lse, "LSE", at::kFloat);
     }
-    void complete(size_t need, at::IntArrayRef lse_shape) {
-        if (!workspace) workspace = at::empty({static_cast<int64_t>(need)}, q.options().dtype(at::kByte));
+    void check_all(at::IntArrayRef lse_shape) const {
         require_like(v, "V", k);
         require_like(o, "O", q);
         require_like(dout, "dO", q);
         if (dq) require_like(*dq, "dQ", q);
-        else dq = at::empty_like(q);
         if (dk) require_like(*dk, "dK", k);
-        else dk = at::empty_like(k);
         if (dv) require_like(*dv, "dV", k);
-        else dv = at::empty_like(k);
         require_like(lse, "LSE", q, lse_shape, at::kFloat);
         // its size is checked by the library (GQA_ERR_WORKSPACE, with the needed size in the error text)
-        TORCH_CHECK_VALUE(workspace->is_cuda() && workspace->device() == q.device() && workspace->is_contiguous(),
-                          "workspace must be contiguous memory on ", q.device());
+        if (workspace)
+            TORCH_CHECK_VALUE(workspace->is_cuda() && workspace->device() == q.device() && workspace->is_contiguous(),
+                              "workspace must be contiguous memory on ", q.device());
+    }
+    void allocate(size_t need, const CallStream& stream) {
+        if (!workspace) workspace = at::empty({static_cast<int64_t>(need)}, q.options().dtype(at::kByte));
+        if (!dq) dq = stream.empty_like(q);
+        if (!dk) dk = stream.empty_like(k);
+        if (!dv) dv = stream.empty_like(k);
     }
 };
 
@@ -201,15 +228,16 @@ Grads backward(BwdTensors t, const CallArgs& a) {
                                     : api.bwd_workspace_bytes_ex(d.B, d.Hq, d.Hkv, d.S, d.D, a.causal,
                                                                  a.bwd_flags & GQA_BWD_SPLIT_HEADS);
     if (need == 0) check_status("gqa_bwd_workspace_bytes", GQA_ERR_UNSUPPORTED);
-    const c10::cuda::CUDAGuard guard(t.q.device());
     const int64_t lse_shape[3] = {d.B, d.Hq, d.S};
-    t.complete(need, lse_shape);
+    t.check_all(lse_shape);
+    const CallStream stream(t.q, a.stream);
+    t.allocate(need, stream);
     const unsigned flags = a.bwd_flags | (a.bshd ? GQA_LAYOUT_BSHD : 0u);
     check_status(flags ? "gqa_bwd_ex" : "gqa_bwd",
                  api.bwd_ex(t.q.data_ptr(), t.k.data_ptr(), t.v.data_ptr(), t.o.data_ptr(), t.dout.data_ptr(),
                             static_cast<const float*>(t.lse.data_ptr()), t.dq->data_ptr(), t.dk->data_ptr(),
                             t.dv->data_ptr(), d.B, d.Hq, d.Hkv, d.S, d.D, a.causal, scale_or_default(a.scale, d.D),
-                            t.workspace->data_ptr(), t.workspace->nbytes(), stream_of(t.q, a.stream), flags));
+                            t.workspace->data_ptr(), t.workspace->nbytes(), stream.handle(), flags));
     return {std::move(*t.dq), std::move(*t.dk), std::move(*t.dv)};
 }
 
@@ -219,15 +247,16 @@ Grads backward_varlen(BwdTensors t, const Tensor& cu, int64_t max_seqlen, const 
     const Dims d = packed_dims(t.q, t.k, cu);
     const size_t need = t.workspace ? 1 : api.bwd_varlen_workspace_bytes(d.S, d.Hq, d.Hkv, d.D);
     if (need == 0) check_status("gqa_bwd_varlen_workspace_bytes", GQA_ERR_UNSUPPORTED);
-    const c10::cuda::CUDAGuard guard(t.q.device());
     const int64_t lse_shape[2] = {d.Hq, d.S};
-    t.complete(need, lse_shape);
+    t.check_all(lse_shape);
+    const CallStream stream(t.q, a.stream);
+    t.allocate(need, stream);
     check_status("gqa_bwd_varlen",
                  api.bwd_varlen(t.q.data_ptr(), t.k.data_ptr(), t.v.data_ptr(), t.o.data_ptr(), t.dout.data_ptr(),
                                 static_cast<const float*>(t.lse.data_ptr()), t.dq->data_ptr(), t.dk->data_ptr(),
                                 t.dv->data_ptr(), static_cast<const int*>(cu.data_ptr()), as_int(cu.numel()) - 1, d.S,
                                 as_int(max_seqlen), d.Hq, d.Hkv, d.D, a.causal, scale_or_default(a.scale, d.D),
-                                t.workspace->data_ptr(), t.workspace->nbytes(), stream_of(t.q, a.stream)));
+                                t.workspace->data_ptr(), t.workspace->nbytes(), stream.handle()));
     return {std::move(*t.dq), std::move(*t.dk), std::move(*t.dv)};
 }
 

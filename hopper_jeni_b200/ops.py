@@ -5,6 +5,10 @@ checks, allocations and launches run in the native binding (csrc/torch_binding.c
 Layouts follow the reference launchers (src/attention/GQA_bwd_baseline.cu:549-554,
 src/attention/GQA_fwd_ref.cu:631-634): Q/O/dO/dQ ``[B,Hq,S,D]``, K/V/dK/dV ``[B,Hkv,S,D]`` bf16
 contiguous, LSE ``[B,Hq,S]`` fp32 (natural log).
+
+``stream``: the stream the kernels run on (default: torch's current one).  What a call allocates belongs to that stream,
+and what it returns is kept from reuse until the caller's current stream is done with it too.  The caller orders the two
+streams (inputs ready before, results read after) and keeps the tensors it passes in alive until the call has run.
 """
 from __future__ import annotations
 
