@@ -346,7 +346,6 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     auto q_z_of = [&](const WorkItem& w, int it) { return p.bshd ? w.b : w.b * p.Hq + head_of(w, it); };
     auto ws_z_of = [&](const WorkItem& w, int it) { return w.b * p.Hq + head_of(w, it); };
 
-    pdl_launch_dependents();
     if (tid == 0) {
         mbar_init(kv_full, 1);
         mbar_init(p_ready, Cfg::kEwThreads);
@@ -423,7 +422,15 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
             for (int j = 0; ok; ++j) {
                 item_slot[j & (kItemSlots - 1)] = idx;
                 mbar_arrive(&item_full[j & (kItemSlots - 1)]);
-                if (idx < 0) break;
+                if (idx < 0) {
+                    // The finalise kernel may come up from here on, under the last tile pairs of every block, and not
+                    // sooner: its waiting blocks take registers on every SM that this launch leaves idle, and a main
+                    // kernel of another stream then finds no SM to run on.  Four streams of B1 Hq8 Hkv2 S2048 D64 (32
+                    // items each), per call of one: 112 us, 229 with the trigger at the start of the block, 117 without
+                    // dependent launches; one stream alone 103.5, 103.4 and 109.
+                    pdl_launch_dependents();
+                    break;
+                }
                 const WorkItem w = decode(idx);
                 if (j > 0) {
                     // a block of this launch that gave up has left a non-zero status word: stop taking items
