@@ -47,6 +47,7 @@ constexpr int kHalf = 64;               // keys per half-block
 constexpr int kFwdThreads = 352;
 constexpr int kWarpTma = 8, kWarpMma0 = 9;
 constexpr int kItemSlots = 2;
+constexpr int kMaxPassedOver = 256;  // empty items of a packed batch that are taken over before one is published
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kRescaleThreshold = 8.0f;  // in log2 units
@@ -138,7 +139,7 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     // Packed variable-length batch: the sequence is a row range [y0, y0 + len) of the one [T, H*D] matrix; rows past
     // its end belong to the next sequence (or read as zeros past T): as keys they are masked like keys beyond S,
     // as queries they are computed and not stored.  The grid covers max_seqlen: an item beyond its sequence has
-    // n_tiles = 0 and no key blocks; a block's own may be such a one, further ones are passed over by the producer.
+    // n_tiles = 0 and no key blocks; the producer passes most of them over, and every role does nothing in one.
     auto decode = [&](int x, int y, int z) -> Item {
         Item w;
         const int idx = p.causal ? (p.n_groups - 1 - x) : x;  // heavy causal tiles first
@@ -226,9 +227,12 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
             tma_prefetch_desc(&mapV);
             uint32_t n_claims = 0;
             int x = blockIdx.x, y = blockIdx.y, z = blockIdx.z;
-            // The next item that has work: x = -1 when there is none.  False: a wait gave up.
+            // The next item: x = -1 when there is none.  False: a wait gave up.  Empty items of a packed batch are passed
+            // over here, at 0.3 to 0.4 us each, while the other roles wait for the next one.  Long runs of them (a batch with many
+            // empty sequences beside a long one) would outlast that wait, so every kMaxPassedOver-th is published: the
+            // roles find nothing to do in it and wait anew, and the look at the status word comes round.
             auto claim = [&]() -> bool {
-                for (;;) {
+                for (int passed_over = 0;; ++passed_over) {
                     mbar_expect_tx(clc_full, 16);
                     clc_try_cancel(clc_answer, clc_full);
                     if (!mbar_wait(clc_full, n_claims & 1, ctx, 15)) return false;
@@ -239,7 +243,7 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                         x = -1;
                         return true;
                     }
-                    if (!p.cu || decode(x, y, z).n_tiles > 0) return true;
+                    if (!p.cu || passed_over >= kMaxPassedOver || decode(x, y, z).n_tiles > 0) return true;
                 }
             };
             bool ok = true;

@@ -74,3 +74,18 @@ def test_items_packed(gqa_lib, D, causal):
         for g in range(Hkv if n else 0):
             h = slice(g * G, (g + 1) * G)
             _check(o[r, h].transpose(0, 1), lse[h, r], q[r, h].transpose(0, 1), k[r, g], v[r, g], scale, causal)
+
+
+@pytest.mark.parametrize("causal", [False, True])
+def test_long_run_of_empty_items(gqa_lib, causal):
+    """65 534 empty sequences in front of one of 32 768 tokens: 7.3 million empty items per SM in a row, about two
+    seconds, and the bounded wait of the other roles lasts one (2e9 cycles), so they must be woken in between."""
+    S, Hq, Hkv, D, n_seqs = 32768, 128, 8, 64, 65535
+    gen = torch.Generator(device="cuda").manual_seed(10)
+    q, k, v = (torch.randn(S, h, D, generator=gen, device="cuda").bfloat16() for h in (Hq, Hkv, Hkv))
+    cu = torch.zeros(n_seqs + 1, dtype=torch.int32, device="cuda")
+    cu[-1] = S
+    o, lse = ops.gqa_forward_varlen(q, k, v, cu, S, causal=causal)
+    ops.check_status()
+    o_ref, lse_ref = ops.gqa_forward(q[None], k[None], v[None], causal=causal, layout="bshd")
+    assert torch.equal(o, o_ref[0]) and torch.equal(lse, lse_ref[0])
