@@ -61,6 +61,7 @@ SELFTEST_EXPORTS = {
     "gqa_checker_fwd_simt": (_i, [_vp, _vp, _vp, _vp, _fp, _i, _i, _i, _i, _i, _i, _f, _vp]),
     "gqa_checker_bwd_simt": (_i, [_vp, _vp, _vp, _vp, _vp, _fp, _vp, _vp, _vp, _fp,
                                   _i, _i, _i, _i, _i, _i, _f, _vp]),
+    "gqa_selftest_refused_launch": (_i, [ctypes.POINTER(_i)]),
     "gqa_selftest_timeout": (_i, [_vp, ctypes.c_longlong, _i, _vp]),
 }
 

@@ -55,7 +55,10 @@ cudaError_t launch_after(void (*kernel)(P...), dim3 grid, unsigned threads, size
     cfg.stream = stream;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    const cudaError_t rc = cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    // left on the thread, the error of a refused launch would be reported by the check behind the next one
+    if (rc != cudaSuccess) (void)cudaGetLastError();
+    return rc;
 }
 
 // SMs of the current device (1 when it cannot be asked).

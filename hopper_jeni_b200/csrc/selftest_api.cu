@@ -89,7 +89,22 @@ __global__ void __launch_bounds__(128, 1) timeout_selftest_kernel(unsigned int* 
     }
 }
 
+__global__ void empty_selftest_kernel() {}
+
+int refused_launch() {
+    GQA_CUDA_TRY(gqa::launch_after(empty_selftest_kernel, dim3(0), 32, 0, nullptr));
+    return GQA_OK;
+}
+
 }  // namespace
+
+extern "C" int gqa_selftest_refused_launch(int* left_behind) {
+    if (!left_behind) return GQA_ERR_BAD_ARGUMENT;
+    (void)cudaGetLastError();
+    const int rc = refused_launch();
+    *left_behind = static_cast<int>(cudaPeekAtLastError());
+    return rc;
+}
 
 extern "C" int gqa_selftest_timeout(void* status_word, long long limit_cycles, int blocks, gqa_stream_t stream_) {
     cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);

@@ -33,6 +33,13 @@ int gqa_selftest_umma(const void* X, const void* Y, float* C, int N, int mode, i
                       gqa_stream_t stream);
 
 /*
+ * A launch that the runtime refuses on the host (an empty grid; nothing runs) through the helper
+ * that the backward's dependent stages are launched with.  Returns its status, GQA_ERR_CUDA, and in
+ * *left_behind the error that it leaves on the calling thread: 0 for none.
+ */
+int gqa_selftest_refused_launch(int* left_behind);
+
+/*
  * Issue-rate probe over arrangements 0-5: reps x 8 back-to-back K = 16 products into one
  * accumulator, issued by one warp or (two_issuers != 0) by two warps on separate accumulators;
  * *cycles_per_product (host memory) receives the SM cycles per product per issuing warp.

@@ -2,6 +2,8 @@
 mode's turn counters itself, and each later stage may start while the one before it still runs.  Calls back to back on one
 workspace, poisoned in front of each, give the same bits (dK, dV; dQ too in the ordered mode) as a call on a fresh one, and
 dQ of the default mode differs by the order of its fp32 sums alone (rounded to bf16: 2^-8 relative, 4e-3 in 2-norm)."""
+import ctypes
+
 import pytest
 import torch
 
@@ -38,3 +40,11 @@ def test_poisoned_workspace_back_to_back(gqa_lib, shape, deterministic):
             assert torch.equal(dq, ref[0])
         else:
             assert (dq.float() - ref[0].float()).norm() <= 4e-3 * ref[0].float().norm() + 1e-12
+
+
+def test_refused_launch_leaves_no_error_behind(selftest_lib):
+    """The launch helper of the dependent stages, given a launch that the runtime refuses on the host (an empty grid): an
+    error left on the thread would be reported by the check behind the next launch, though that one is good."""
+    left = ctypes.c_int(-1)
+    assert selftest_lib.gqa_selftest_refused_launch(ctypes.byref(left)) == -4  # GQA_ERR_CUDA
+    assert left.value == 0
