@@ -101,16 +101,60 @@ float scale_or_default(double scale, int D) {  // NaN: not given
     return static_cast<float>(std::isnan(scale) ? 1.0 / std::sqrt(static_cast<double>(D)) : scale);
 }
 
+struct CallArgs {
+    bool causal = false, bshd = false;
+    double scale = std::nan("");
+    unsigned bwd_flags = 0;                 // GQA_BWD_* of a backward call
+    std::optional<uintptr_t> stream;
+    bool subclass = false;                  // Q, K or V is of a subclass of torch.Tensor
+};
+
+// No autograd bookkeeping for the outputs, they are plain memory; not around what a subclass overrides.
+struct PlainMemory {
+    explicit PlainMemory(const CallArgs& a) {
+        if (!a.subclass) below_.emplace();
+    }
+    std::optional<at::AutoDispatchBelowADInplaceOrView> below_;
+};
+
+// For a subclass of torch.Tensor: outputs are made through torch.empty_like (and contiguous copies through the method),
+// so that they are of the subclass and its overrides are heard.  C++ knows neither.
+Tensor unpack_result(PyObject* r) {
+    if (!r) {
+        python_error e;
+        e.persist();
+        throw std::move(e);
+    }
+    const auto owned = pybind11::reinterpret_steal<pybind11::object>(r);
+    TORCH_CHECK_TYPE(THPVariable_Check(r), "expected a torch.Tensor, got ", Py_TYPE(r)->tp_name);
+    return THPVariable_Unpack(r);
+}
+Tensor py_empty_like(const Tensor& t) {
+    pybind11::gil_scoped_acquire gil;
+    const auto self = pybind11::reinterpret_steal<pybind11::object>(THPVariable_Wrap(t));
+    const auto torch = pybind11::reinterpret_steal<pybind11::object>(PyImport_ImportModule("torch"));
+    return unpack_result(torch ? PyObject_CallMethod(torch.ptr(), "empty_like", "O", self.ptr()) : nullptr);
+}
+Tensor contiguous(const Tensor& t, const CallArgs& a) {
+    if (!a.subclass || t.is_contiguous()) return t.contiguous();
+    pybind11::gil_scoped_acquire gil;
+    const auto self = pybind11::reinterpret_steal<pybind11::object>(THPVariable_Wrap(t));
+    return unpack_result(PyObject_CallMethod(self.ptr(), "contiguous", nullptr));
+}
+
 // The device and the stream of one call, current for as long as this lives.  A stream that was given and is not the
 // caller's current one owns what the call allocates: torch's allocator orders the reuse of a block by its stream, so a
 // workspace taken from the current stream's pool could be handed out again, and an output could be memory that the
 // current stream still uses, while the kernels run on the given one.
 class CallStream {
 public:
-    CallStream(const Tensor& q, const std::optional<uintptr_t>& given)
-        : device_(q.device()), caller_(c10::cuda::getCurrentCUDAStream(q.get_device())), handle_(caller_.stream()) {
-        if (!given || reinterpret_cast<cudaStream_t>(*given) == caller_.stream()) return;
-        const auto run = c10::cuda::getStreamFromExternal(reinterpret_cast<cudaStream_t>(*given), q.get_device());
+    CallStream(const Tensor& q, const CallArgs& a)
+        : device_(q.device()),
+          caller_(c10::cuda::getCurrentCUDAStream(q.get_device())),
+          handle_(caller_.stream()),
+          subclass_(a.subclass) {
+        if (!a.stream || reinterpret_cast<cudaStream_t>(*a.stream) == caller_.stream()) return;
+        const auto run = c10::cuda::getStreamFromExternal(reinterpret_cast<cudaStream_t>(*a.stream), q.get_device());
         handle_ = run.stream();
         given_.emplace(run);
     }
@@ -120,7 +164,12 @@ public:
         if (given_) t.record_stream(caller_.unwrap());
         return t;
     }
-    Tensor empty_like(const Tensor& t) const { return returned(at::empty_like(t)); }
+    Tensor empty_like(const Tensor& t, const char* name) const {
+        if (!subclass_) return returned(at::empty_like(t));
+        Tensor r = py_empty_like(t);
+        require_like(r, name, t);  // an override may have returned anything
+        return returned(std::move(r));
+    }
     Tensor empty_f32(const Tensor& like, at::IntArrayRef shape) const {
         return returned(at::empty(shape, like.options().dtype(at::kFloat)));
     }
@@ -129,14 +178,8 @@ private:
     const c10::cuda::CUDAGuard device_;
     const c10::cuda::CUDAStream caller_;
     gqa_stream_t handle_;
+    const bool subclass_;
     std::optional<c10::cuda::CUDAStreamGuard> given_;
-};
-
-struct CallArgs {
-    bool causal = false, bshd = false;
-    double scale = std::nan("");
-    unsigned bwd_flags = 0;                 // GQA_BWD_* of a backward call
-    std::optional<uintptr_t> stream;
 };
 
 void check_qkv(const Tensor& q, const Tensor& k, const Tensor& v) {
@@ -147,15 +190,15 @@ void check_qkv(const Tensor& q, const Tensor& k, const Tensor& v) {
 
 std::tuple<Tensor, Tensor> forward(const Tensor& q, const Tensor& k, const Tensor& v, const CallArgs& a, OptTensor out,
                                    OptTensor lse) {
-    at::AutoDispatchBelowADInplaceOrView below;  // plain memory: no autograd bookkeeping for the outputs
+    const PlainMemory below(a);
     check_qkv(q, k, v);
     const Dims d = dims(q, k, a.bshd);
     require_like(v, "V", k);
     const int64_t lse_shape[3] = {d.B, d.Hq, d.S};
     if (out) require_like(*out, "O", q);
     if (lse) require_like(*lse, "LSE", q, lse_shape, at::kFloat);
-    const CallStream stream(q, a.stream);
-    if (!out) out = stream.empty_like(q);
+    const CallStream stream(q, a);
+    if (!out) out = stream.empty_like(q, "O");
     if (!lse) lse = stream.empty_f32(q, lse_shape);
     check_status("gqa_fwd_ex", api.fwd_ex(q.data_ptr(), k.data_ptr(), v.data_ptr(), out->data_ptr(),
                                           static_cast<float*>(lse->data_ptr()), d.B, d.Hq, d.Hkv, d.S, d.D, a.causal,
@@ -166,15 +209,15 @@ std::tuple<Tensor, Tensor> forward(const Tensor& q, const Tensor& k, const Tenso
 
 std::tuple<Tensor, Tensor> forward_varlen(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu,
                                           int64_t max_seqlen, const CallArgs& a, OptTensor out, OptTensor lse) {
-    at::AutoDispatchBelowADInplaceOrView below;
+    const PlainMemory below(a);
     check_qkv(q, k, v);
     const Dims d = packed_dims(q, k, cu);
     require_like(v, "V", k);
     const int64_t lse_shape[2] = {d.Hq, d.S};
     if (out) require_like(*out, "O", q);
     if (lse) require_like(*lse, "LSE", q, lse_shape, at::kFloat);
-    const CallStream stream(q, a.stream);
-    if (!out) out = stream.empty_like(q);
+    const CallStream stream(q, a);
+    if (!out) out = stream.empty_like(q, "O");
     if (!lse) lse = stream.empty_f32(q, lse_shape);
     check_status("gqa_fwd_varlen",
                  api.fwd_varlen(q.data_ptr(), k.data_ptr(), v.data_ptr(), out->data_ptr(),
@@ -214,14 +257,14 @@ struct BwdTensors {
     }
     void allocate(size_t need, const CallStream& stream) {
         if (!workspace) workspace = at::empty({static_cast<int64_t>(need)}, q.options().dtype(at::kByte));
-        if (!dq) dq = stream.empty_like(q);
-        if (!dk) dk = stream.empty_like(k);
-        if (!dv) dv = stream.empty_like(k);
+        if (!dq) dq = stream.empty_like(q, "dQ");
+        if (!dk) dk = stream.empty_like(k, "dK");
+        if (!dv) dv = stream.empty_like(v, "dV");
     }
 };
 
 Grads backward(BwdTensors t, const CallArgs& a) {
-    at::AutoDispatchBelowADInplaceOrView below;
+    const PlainMemory below(a);
     t.check_inputs();
     const Dims d = dims(t.q, t.k, a.bshd);
     const size_t need = t.workspace ? 1
@@ -230,7 +273,7 @@ Grads backward(BwdTensors t, const CallArgs& a) {
     if (need == 0) check_status("gqa_bwd_workspace_bytes", GQA_ERR_UNSUPPORTED);
     const int64_t lse_shape[3] = {d.B, d.Hq, d.S};
     t.check_all(lse_shape);
-    const CallStream stream(t.q, a.stream);
+    const CallStream stream(t.q, a);
     t.allocate(need, stream);
     const unsigned flags = a.bwd_flags | (a.bshd ? GQA_LAYOUT_BSHD : 0u);
     check_status(flags ? "gqa_bwd_ex" : "gqa_bwd",
@@ -242,14 +285,14 @@ Grads backward(BwdTensors t, const CallArgs& a) {
 }
 
 Grads backward_varlen(BwdTensors t, const Tensor& cu, int64_t max_seqlen, const CallArgs& a) {
-    at::AutoDispatchBelowADInplaceOrView below;
+    const PlainMemory below(a);
     t.check_inputs();
     const Dims d = packed_dims(t.q, t.k, cu);
     const size_t need = t.workspace ? 1 : api.bwd_varlen_workspace_bytes(d.S, d.Hq, d.Hkv, d.D);
     if (need == 0) check_status("gqa_bwd_varlen_workspace_bytes", GQA_ERR_UNSUPPORTED);
     const int64_t lse_shape[2] = {d.Hq, d.S};
     t.check_all(lse_shape);
-    const CallStream stream(t.q, a.stream);
+    const CallStream stream(t.q, a);
     t.allocate(need, stream);
     check_status("gqa_bwd_varlen",
                  api.bwd_varlen(t.q.data_ptr(), t.k.data_ptr(), t.v.data_ptr(), t.o.data_ptr(), t.dout.data_ptr(),
@@ -266,14 +309,15 @@ using torch::autograd::variable_list;
 
 struct Attention : torch::autograd::Function<Attention> {
     static Tensor forward(AutogradContext* ctx, Tensor q, Tensor k, Tensor v, const CallArgs& a) {
-        q = q.contiguous();
-        k = k.contiguous();
-        v = v.contiguous();
+        q = contiguous(q, a);
+        k = contiguous(k, a);
+        v = contiguous(v, a);
         auto [o, lse] = ::forward(q, k, v, a, std::nullopt, std::nullopt);
         ctx->save_for_backward({q, k, v, o, lse});
         ctx->saved_data["causal"] = a.causal;
         ctx->saved_data["bshd"] = a.bshd;
         ctx->saved_data["scale"] = a.scale;
+        ctx->saved_data["subclass"] = a.subclass;
         ctx->saved_data["flags"] = static_cast<int64_t>(a.bwd_flags);
         return o;
     }
@@ -283,6 +327,7 @@ struct Attention : torch::autograd::Function<Attention> {
         a.causal = ctx->saved_data["causal"].toBool();
         a.bshd = ctx->saved_data["bshd"].toBool();
         a.scale = ctx->saved_data["scale"].toDouble();
+        a.subclass = ctx->saved_data["subclass"].toBool();
         a.bwd_flags = static_cast<unsigned>(ctx->saved_data["flags"].toInt());
         const Tensor dout = grads[0].contiguous();
         Grads g = ::backward({s[0], s[1], s[2], s[3], dout, s[4], {}, {}, {}, {}}, a);
@@ -293,13 +338,14 @@ struct Attention : torch::autograd::Function<Attention> {
 struct AttentionVarlen : torch::autograd::Function<AttentionVarlen> {
     static Tensor forward(AutogradContext* ctx, Tensor q, Tensor k, Tensor v, const Tensor& cu, int64_t max_seqlen,
                           const CallArgs& a) {
-        q = q.contiguous();
-        k = k.contiguous();
-        v = v.contiguous();
+        q = contiguous(q, a);
+        k = contiguous(k, a);
+        v = contiguous(v, a);
         auto [o, lse] = ::forward_varlen(q, k, v, cu, max_seqlen, a, std::nullopt, std::nullopt);
         ctx->save_for_backward({q, k, v, o, lse, cu});
         ctx->saved_data["causal"] = a.causal;
         ctx->saved_data["scale"] = a.scale;
+        ctx->saved_data["subclass"] = a.subclass;
         ctx->saved_data["max_seqlen"] = max_seqlen;
         return o;
     }
@@ -308,6 +354,7 @@ struct AttentionVarlen : torch::autograd::Function<AttentionVarlen> {
         CallArgs a;
         a.causal = ctx->saved_data["causal"].toBool();
         a.scale = ctx->saved_data["scale"].toDouble();
+        a.subclass = ctx->saved_data["subclass"].toBool();
         const Tensor dout = grads[0].contiguous();
         Grads g = ::backward_varlen({s[0], s[1], s[2], s[3], dout, s[4], {}, {}, {}, {}}, s[5],
                                     ctx->saved_data["max_seqlen"].toInt(), a);
@@ -323,6 +370,10 @@ const Tensor& tensor_arg(PyObject* o, const char* name) {
 OptTensor opt_tensor_arg(PyObject* o, const char* name) {
     if (o == Py_None) return std::nullopt;
     return tensor_arg(o, name);
+}
+bool subclass_arg(PyObject* q, PyObject* k, PyObject* v) {  // (a Parameter counts as a plain tensor)
+    return !(THPVariable_CheckTypeExact(Py_TYPE(q)) && THPVariable_CheckTypeExact(Py_TYPE(k)) &&
+             THPVariable_CheckTypeExact(Py_TYPE(v)));
 }
 bool bool_arg(PyObject* o) {
     const int r = PyObject_IsTrue(o);
@@ -372,6 +423,7 @@ PyObject* py_forward(PyObject*, PyObject* const* x, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     count_args(n, 9);
     CallArgs a;
+    a.subclass = subclass_arg(x[0], x[1], x[2]);
     a.causal = bool_arg(x[3]);
     a.scale = scale_arg(x[4]);
     a.stream = stream_arg(x[7]);
@@ -392,6 +444,7 @@ PyObject* py_backward(PyObject*, PyObject* const* x, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     count_args(n, 15);
     CallArgs a;
+    a.subclass = subclass_arg(x[0], x[1], x[2]);
     a.causal = bool_arg(x[6]);
     a.scale = scale_arg(x[7]);
     a.stream = stream_arg(x[12]);
@@ -414,6 +467,7 @@ PyObject* py_forward_varlen(PyObject*, PyObject* const* x, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     count_args(n, 10);
     CallArgs a;
+    a.subclass = subclass_arg(x[0], x[1], x[2]);
     a.causal = bool_arg(x[5]);
     a.scale = scale_arg(x[6]);
     a.stream = stream_arg(x[9]);
@@ -435,6 +489,7 @@ PyObject* py_backward_varlen(PyObject*, PyObject* const* x, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     count_args(n, 15);
     CallArgs a;
+    a.subclass = subclass_arg(x[0], x[1], x[2]);
     a.causal = bool_arg(x[8]);
     a.scale = scale_arg(x[9]);
     a.stream = stream_arg(x[14]);
@@ -457,6 +512,7 @@ PyObject* py_attention(PyObject*, PyObject* const* x, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     count_args(n, 7);
     CallArgs a;
+    a.subclass = subclass_arg(x[0], x[1], x[2]);
     a.causal = bool_arg(x[3]);
     a.scale = scale_arg(x[4]);
     a.bshd = layout_arg(x[5]);
@@ -476,6 +532,7 @@ PyObject* py_attention_varlen(PyObject*, PyObject* const* x, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     count_args(n, 7);
     CallArgs a;
+    a.subclass = subclass_arg(x[0], x[1], x[2]);
     a.causal = bool_arg(x[5]);
     a.scale = scale_arg(x[6]);
     const Tensor &q = tensor_arg(x[0], "Q"), &k = tensor_arg(x[1], "K"), &v = tensor_arg(x[2], "V"),
