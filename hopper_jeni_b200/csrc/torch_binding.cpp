@@ -382,8 +382,9 @@ bool bool_arg(PyObject* o) {
 }
 double scale_arg(PyObject* o) {
     if (o == Py_None) return std::nan("");
-    const double v = PyFloat_AsDouble(o);
-    if (v == -1.0 && PyErr_Occurred()) throw python_error();
+    const auto f = pybind11::reinterpret_steal<pybind11::object>(PyNumber_Float(o));  // whatever float() takes
+    if (!f) throw python_error();
+    const double v = PyFloat_AS_DOUBLE(f.ptr());
     return std::isnan(v) ? 0.0 : v;  // NaN marks "not given" above; the library refuses both
 }
 int64_t int_arg(PyObject* o) {

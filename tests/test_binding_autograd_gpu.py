@@ -1,4 +1,8 @@
-"""GPU tests of what the native host path owes torch besides numbers: the classes of its outputs."""
+"""GPU tests of what the native host path owes its callers besides numbers: the classes of its outputs, the forms in which
+it takes its arguments."""
+import fractions
+
+import numpy as np
 import pytest
 import torch
 
@@ -80,3 +84,13 @@ def test_output_of_an_override_is_checked(gqa_lib):
     q, k, v, _ = (t.as_subclass(WrongShape) for t in _inputs(False))
     with pytest.raises(ValueError, match="O has shape"):
         ops.gqa_forward(q, k, v)
+
+
+@pytest.mark.parametrize("scale", [np.float32(0.125), fractions.Fraction(1, 8), "0.125", torch.tensor(0.125)])
+def test_scale_is_whatever_float_takes(gqa_lib, scale):
+    q, k, v, do = _inputs(False)
+    o, lse = ops.gqa_forward(q, k, v, scale=0.125)
+    assert torch.equal(ops.gqa_forward(q, k, v, scale=scale)[0], o)
+    assert torch.equal(gqa_attention(q, k, v, scale=scale), o)
+    assert torch.equal(ops.gqa_backward(q, k, v, o, do, lse, scale=scale)[1],
+                       ops.gqa_backward(q, k, v, o, do, lse, scale=0.125)[1])
