@@ -276,7 +276,7 @@ Grads backward(BwdTensors t, const CallArgs& a) {
     const CallStream stream(t.q, a);
     t.allocate(need, stream);
     const unsigned flags = a.bwd_flags | (a.bshd ? GQA_LAYOUT_BSHD : 0u);
-    check_status(flags ? "gqa_bwd_ex" : "gqa_bwd",
+    check_status("gqa_bwd_ex",
                  api.bwd_ex(t.q.data_ptr(), t.k.data_ptr(), t.v.data_ptr(), t.o.data_ptr(), t.dout.data_ptr(),
                             static_cast<const float*>(t.lse.data_ptr()), t.dq->data_ptr(), t.dk->data_ptr(),
                             t.dv->data_ptr(), d.B, d.Hq, d.Hkv, d.S, d.D, a.causal, scale_or_default(a.scale, d.D),

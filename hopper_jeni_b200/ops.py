@@ -38,14 +38,7 @@ def _req(t: torch.Tensor, name: str, dtype) -> None:
         raise ValueError(f"{name} must be contiguous")
 
 
-def _dims(q, k, layout="bhsd"):
-    if layout == "bshd":
-        B, S, Hq, D = q.shape
-        if k.shape[0] != B or k.shape[1] != S or k.shape[3] != D:
-            raise ValueError(f"K/V shape {tuple(k.shape)} does not match Q {tuple(q.shape)}")
-        return B, Hq, k.shape[2], S, D
-    if layout != "bhsd":
-        raise ValueError(f"layout must be 'bhsd' or 'bshd', got {layout!r}")
+def _dims(q, k):
     B, Hq, S, D = q.shape
     if k.shape[0] != B or k.shape[2] != S or k.shape[3] != D:
         raise ValueError(f"K/V shape {tuple(k.shape)} does not match Q {tuple(q.shape)}")

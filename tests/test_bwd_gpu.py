@@ -146,3 +146,32 @@ def test_backward_rejects_small_workspace(gqa_lib):
     with pytest.raises(capi.GqaError) as e:
         ops.gqa_backward(q, q, q, q, q, lse, workspace=ws)
     assert e.value.status == -3
+
+
+def test_plain_entry_points_give_the_extended_ones_bits(gqa_lib):
+    """gqa_fwd and gqa_bwd through ctypes (the Python operators go through gqa_fwd_ex and gqa_bwd_ex): the same O, LSE, dK
+    and dV, and dQ up to the order of its fp32 reductions (rounded to bf16: 2^-8)."""
+    B, Hq, Hkv, S, D = 2, 4, 2, 300, 64
+    q, k, v, do = (util.to_dev_bf16(x) for x in util.make_inputs(B, Hq, Hkv, S, D, seed=43))
+    sc = util.default_scale(D)
+    o_ref, lse_ref = ops.gqa_forward(q, k, v, causal=True, scale=sc)
+    dq_ref, dk_ref, dv_ref = ops.gqa_backward(q, k, v, o_ref, do, lse_ref, causal=True, scale=sc)
+    o, dq, dk, dv = (torch.full_like(t, float("nan")) for t in (q, q, k, v))
+    lse = torch.full_like(lse_ref, float("nan"))
+    ws = torch.empty(ops.bwd_workspace_bytes(B, Hq, Hkv, S, D, True), dtype=torch.uint8, device="cuda")
+    stream = int(torch.cuda.current_stream().cuda_stream)
+    dims = (B, Hq, Hkv, S, D, 1, sc)
+    assert gqa_lib.gqa_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), *dims, stream) == 0
+    assert gqa_lib.gqa_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse.data_ptr(),
+                           dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), *dims, ws.data_ptr(), ws.numel(), stream) == 0
+    ops.check_status(ws)
+    for got, ref in ((o, o_ref), (lse, lse_ref), (dk, dk_ref), (dv, dv_ref)):
+        assert torch.equal(got, ref)
+    assert (dq.float() - dq_ref.float()).norm() <= 4e-3 * dq_ref.float().norm()
+
+
+def test_refused_backward_names_the_function_that_refused(gqa_lib):
+    q, k, v, do = (util.to_dev_bf16(x) for x in util.make_inputs(1, 2, 1, 128, 64, seed=44))
+    o, lse = ops.gqa_forward(q, k, v)
+    with pytest.raises(capi.GqaError, match="gqa_bwd_ex failed with GQA_ERR_WORKSPACE"):
+        ops.gqa_backward(q, k, v, o, do, lse, workspace=torch.empty(256, dtype=torch.uint8, device="cuda"))
