@@ -1,12 +1,13 @@
 """GPU tests of what the native host path owes its callers besides numbers: the classes of its outputs, the forms in which
-it takes its arguments."""
+it takes its arguments, errors raised in the autograd engine's thread, calls from several threads."""
 import fractions
+import threading
 
 import numpy as np
 import pytest
 import torch
 
-from hopper_jeni_b200 import ops
+from hopper_jeni_b200 import capi, ops
 from hopper_jeni_b200.autograd import gqa_attention, gqa_attention_varlen
 
 pytestmark = pytest.mark.gpu
@@ -94,3 +95,63 @@ def test_scale_is_whatever_float_takes(gqa_lib, scale):
     assert torch.equal(gqa_attention(q, k, v, scale=scale), o)
     assert torch.equal(ops.gqa_backward(q, k, v, o, do, lse, scale=scale)[1],
                        ops.gqa_backward(q, k, v, o, do, lse, scale=0.125)[1])
+
+
+def _misaligned(t):
+    """The same values two bytes off a 16-byte boundary: contiguous, and refused by the library on the host."""
+    return torch.cat([t.new_zeros(1), t.flatten()])[1:].view(t.shape)
+
+
+@pytest.mark.parametrize("packed", [False, True])
+@pytest.mark.parametrize("unpack,error,words", [
+    (lambda t: t[..., :8], ValueError, "must be contiguous"),                            # refused by the binding
+    (_misaligned, capi.GqaError, "gqa_bwd.* failed with GQA_ERR_BAD_ARGUMENT"),          # refused by the library
+])
+def test_error_in_the_backward_node(gqa_lib, packed, unpack, error, words):
+    """The node runs in the engine's thread; its error reaches the caller, and the next call is good."""
+    q, k, v, do = _inputs(packed)
+    _, _, att = _entry_points(packed)
+    leaves = [t.requires_grad_(True) for t in (q, k, v)]
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: unpack(t) if t.dtype == torch.bfloat16 else t):
+        out = att(*leaves)
+    with pytest.raises(error, match=words):
+        torch.autograd.grad(out, leaves, do)
+    ref = torch.autograd.grad(att(*leaves), leaves, do)
+    assert all(torch.isfinite(g.float()).all() for g in ref)
+
+
+@pytest.mark.parametrize("packed", [False, True])
+def test_threads_with_streams_of_their_own(gqa_lib, packed):
+    """Four threads, each with its own inputs and stream: every call runs on the calling thread's current stream, in the
+    backward on the forward's, and gives the bits of a call made alone."""
+    fwd, _, att = _entry_points(packed)
+    data = [_inputs(packed, seed=50 + i) for i in range(4)]
+
+    def step(i):
+        leaves = [t.clone().requires_grad_(True) for t in data[i][:3]]
+        out = att(*leaves)
+        return [out.detach(), *torch.autograd.grad(out, leaves, data[i][3])[1:], fwd(*data[i][:3])[1]]
+
+    ref = [step(i) for i in range(4)]
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(i):
+        try:
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream):
+                for _ in range(25):
+                    got = step(i)
+                    stream.synchronize()
+                    if not all(torch.equal(a, b) for a, b in zip(got, ref[i])):
+                        bad.append((i, "differs"))
+        except Exception as e:  # noqa: BLE001 (reported below)
+            bad.append((i, e))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join(timeout=60)
+    assert not bad and not any(t.is_alive() for t in threads), bad
+    ops.check_status()

@@ -45,3 +45,47 @@ def test_k_and_v_on_another_device_are_refused(gqa_lib, entry):
     packed = [_fake(T, HKV, D, device="cuda:1") for _ in range(2)]
     with pytest.raises(ValueError, match="K is on cuda:1, expected cuda:0"):
         dict(_calls(kv=kv, packed_kv=packed))[entry]()
+
+
+def _wrong(kind, shape, dtype):
+    """A tensor that differs from what is wanted in one point, and the words of the refusal."""
+    if kind == "shape":
+        return _fake(*shape[:-1], shape[-1] - 1, dtype=dtype), "has shape"
+    if kind == "dtype":
+        return _fake(*shape, dtype=torch.float16), "must be"
+    if kind == "device":
+        return _fake(*shape, dtype=dtype, device="cuda:1"), "is on cuda:1"
+    if kind == "cpu":
+        return _fake(*shape, dtype=dtype, device="cpu"), "must be a CUDA tensor"
+    return _fake(*reversed(shape), dtype=dtype).permute(*reversed(range(len(shape)))), "must be contiguous"
+
+
+BF16, F32 = torch.bfloat16, torch.float32
+GIVEN = {  # the tensors that a call writes into: name of the argument -> (name in the error, shape, type)
+    "forward": {"out": ("O", (B, HQ, S, D), BF16), "lse": ("LSE", (B, HQ, S), F32)},
+    "backward": {"dq": ("dQ", (B, HQ, S, D), BF16), "dk": ("dK", (B, HKV, S, D), BF16), "dv": ("dV", (B, HKV, S, D), BF16)},
+    "forward_varlen": {"out": ("O", (T, HQ, D), BF16), "lse": ("LSE", (HQ, T), F32)},
+    "backward_varlen": {"dq": ("dQ", (T, HQ, D), BF16), "dk": ("dK", (T, HKV, D), BF16), "dv": ("dV", (T, HKV, D), BF16)},
+}
+
+
+@pytest.mark.parametrize("kind", ["shape", "dtype", "device", "cpu", "stride"])
+@pytest.mark.parametrize("entry", GIVEN)
+def test_given_outputs_are_checked(gqa_lib, entry, kind):
+    """The library gets raw pointers: these checks keep its stores inside the tensors."""
+    call = dict(_calls())[entry]
+    for arg, (name, shape, dtype) in GIVEN[entry].items():
+        t, words = _wrong(kind, shape, dtype)
+        with pytest.raises(ValueError, match=f"^{name} {words}"):
+            call(**{arg: t})
+
+
+@pytest.mark.parametrize("entry", ["backward", "backward_varlen"])
+def test_given_workspace_is_checked(gqa_lib, entry):
+    u8 = torch.uint8
+    for ws in (_fake(1 << 20, dtype=u8, device="cpu"), _fake(1 << 20, dtype=u8, device="cuda:1"),
+               _fake(1 << 10, 1 << 10, dtype=u8).t()):
+        with pytest.raises(ValueError, match="workspace must be contiguous memory on cuda:0"):
+            dict(_calls())[entry](workspace=ws)
+    with pytest.raises(TypeError, match="workspace must be a torch.Tensor"):
+        dict(_calls())[entry](workspace=4096)
