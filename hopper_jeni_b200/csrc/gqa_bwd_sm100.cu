@@ -152,9 +152,10 @@ struct BwdCfg {
     static constexpr bool kPAliasesS = (D != 64);
     static constexpr bool kDqAliasesDp = (D != 64);
     // dQ before dK where dQ sits in the dP^T columns: the loop dP^T -> dS^T -> dQ -> drain -> next dP^T then does not
-    // contain dK, which runs while the drain warps empty the columns.  B200, dK first -> dQ first: B4 Hq32 Hkv8 S8192 D128
-    // causal 5 499 -> 5 248 us, B8 Hq12 Hkv4 S4096 D128 2 061 -> 1 984 us, B2 Hq24 S4096 D128 causal with ordered dQ
-    // 865 -> 842 us.  (At D = 64 dQ has columns of its own and the next dP^T waits for dK instead.)
+    // contain dK, which runs while the drain warps empty the columns.  B200, dK first -> dQ first, whole call, medians of
+    // eight runs back to back in four processes of each in turn: B4 Hq32 Hkv8 S8192 D128 causal 5 717 -> 5 633 us, B8 Hq12
+    // Hkv4 S4096 D128 2 158 -> 2 080 us, B2 Hq24 Hkv8 S4096 D128 causal with ordered dQ 852 -> 833 us, B2 Hq32 Hkv8 S1537
+    // D128 causal 166.2 -> 163.5 us.  (At D = 64 dQ has columns of its own and the next dP^T waits for dK instead.)
     static constexpr bool kDqFirst = kDqAliasesDp;
     // D = 64: dS^T is also stored as bf16 over the first half of each warpgroup's dP^T columns, so that dK reads
     // its A operand from TMEM instead of shared memory (shared-memory bandwidth is what bounds this kernel).

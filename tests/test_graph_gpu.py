@@ -1,7 +1,6 @@
 """GPU test: a forward + backward pair captured into a CUDA graph and replayed.  Everything the operators enqueue is
-stream work (a memset node and kernels; tensor maps are encoded on the host at capture time), so a training loop can
-put them into a graph; the backward's work counter and status word are reset by the captured memset at every
-replay."""
+stream work (kernels only; tensor maps are encoded on the host at capture time), so a training loop can put them into a
+graph; the backward's work counter and status word are zeroed by its preprocess kernel at every replay."""
 import pytest
 import torch
 
