@@ -84,7 +84,7 @@ def test_given_stream_is_the_one_that_runs(gqa_lib):
     side = torch.cuda.Stream()
     side.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(side):
-        torch.cuda._sleep(SLEEP)
+        torch.cuda._sleep(5 * SLEEP)
     got = call(stream=side, out=out, lse=lse)
     assert got[0] is out and got[1] is lse
     assert not side.query()
