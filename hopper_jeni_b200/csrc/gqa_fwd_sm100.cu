@@ -1,10 +1,10 @@
 // GQA forward for sm_100a: O = softmax(scale * Q K^T [+ causal]) V, LSE.
 //
-// A work item is two 128-row query tiles (one in short launches, see kSplit) of one (batch, query
+// A work item is two 128-row query tiles (one, where every tile gets an SM of its own) of one (batch, query
 // head); the KV head's 128-row key/value blocks stream through a TMA ring.  A thread block works through
 // several items (see the work-item comment).  Roles:
 //   warps 0-3  softmax warpgroup for query tile 0 (thread = query row = TMEM lane)
-//   warps 4-7  softmax warpgroup for query tile 1 (or for every other key block of the one tile)
+//   warps 4-7  softmax warpgroup for query tile 1
 //   warp  8    TMA producer (Q once per item, K and V rings) and taker of further items
 //   warps 9,10 UMMA issuers, one per query tile: S = Q K^T and O += P V (P read from TMEM)
 // Every key block is handled as two half-blocks of 64 keys, and the 128 fp32 S columns of a tile are two
@@ -66,12 +66,11 @@ struct FwdCfg {
     static constexpr int kSmemKV = 2 * kStages * kTileBytes;
     static constexpr int kBarBytes = 512;
     static constexpr int kSmemTotal = kSmemQ + kSmemKV + kBarBytes;  // the dynamic window must start 1024-byte aligned (checked)
-    static constexpr int kOffMerge = kSmemTotal;                     // kSplit: [2][128] maximum and sum of a row, two barriers
-    static constexpr int kOffList = kOffMerge + 2 * kTile * 8 + 16;  // packed batches: the work list
+    static constexpr int kOffList = kSmemTotal;  // packed batches: the work list
     static constexpr uint32_t kTmemCols = 512;
     static constexpr uint32_t kColS0 = 0, kColS1 = 128, kColO0 = 256, kColO1 = 256 + D;
     static_assert(256 + 2 * D <= 512, "TMEM budget");
-    static_assert(kOffList + (int)sizeof(PackedList) <= 227 * 1024, "shared memory budget");
+    static_assert(kSmemTotal + (int)sizeof(PackedList) <= 227 * 1024, "shared memory budget");
     static_assert(kSmemTotal > 114 * 1024, "one CTA per SM is assumed by the 512-column TMEM allocation");
 };
 
@@ -98,10 +97,7 @@ enum Form {
 // kMore: the launch has more items than SMs, so blocks ask for further ones; without it the kernel is the plain
 // one-item-per-block form (every running count below is a constant 0 there): a launch of the kMore form that has nothing to
 // hand out is 1.5 us slower at B1 Hq4 S128 D64 (8.2 against 6.7 us) and 3 % at B2 Hq12 S1000 D128.
-//
-// kSplit: an item is one query tile, and the two warpgroups take every other key block of it: two streams with an accumulator
-// of their own, merged in the epilogue with the weights that their maxima and sums give them.
-template <int D, Form kForm, bool kMore, bool kSplit>
+template <int D, Form kForm, bool kMore>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                      const __grid_constant__ CUtensorMap mapV, const FwdParams p) {
@@ -137,10 +133,6 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(clc_answer + 16 + kItemSlots * 16);
     volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(tmem_slot + 1);
     static_assert(kBars * 8 + 16 + kItemSlots * 16 + 8 <= Cfg::kBarBytes, "barrier area");
-
-    // kSplit: the rows' maxima and sums, and per warpgroup a barrier that says that they are there
-    float2* ml = reinterpret_cast<float2*>(smem + Cfg::kOffMerge);  // [2][kTile]
-    [[maybe_unused]] uint64_t* merge_full = reinterpret_cast<uint64_t*>(ml + 2 * kTile);
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
@@ -198,10 +190,6 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
         w.n_blk0 = (w.n_tiles == 0) ? 0 : p.causal ? (w.q0 / kTile + 1) : n_blocks_all;
         w.n_blk1 = (w.n_tiles == 2) ? (p.causal ? (w.q0 / kTile + 2) : n_blocks_all) : 0;
         w.n_max = max(w.n_blk0, w.n_blk1);
-        if constexpr (kSplit) {  // the two streams of the one tile
-            w.n_blk1 = w.n_max / 2;
-            w.n_blk0 = w.n_max - w.n_blk1;
-        }
         return w;
     };
     // The j-th item of this block, published by the producer; false = no more (or give up).  In the plain form every role
@@ -225,10 +213,9 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     if (tid == 0) {
         for (int i = 0; i < 2; ++i) {
             mbar_init(&q_full[i], 1);
-            mbar_init(&q_empty[i], kSplit ? 2 : 1);
+            mbar_init(&q_empty[i], 1);
             mbar_init(&o_full[i], 1);
-            mbar_init(&o_empty[i], kSplit ? 256 : 128);
-            if constexpr (kSplit) mbar_init(&merge_full[i], 128);
+            mbar_init(&o_empty[i], 128);
         }
         for (int i = 0; i < 4; ++i) {
             mbar_init(&s_full[i], 1);
@@ -237,10 +224,9 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
         }
         for (int i = 0; i < Cfg::kStages; ++i) {
             mbar_init(&k_full[i], 1);
-            // both issuers release every block, also one they do not use (kSplit: every block has one user)
-            mbar_init(&k_empty[i], kSplit ? 1 : 2);
+            mbar_init(&k_empty[i], 2);  // both issuers release every block, also one they do not use
             mbar_init(&v_full[i], 1);
-            mbar_init(&v_empty[i], kSplit ? 1 : 2);
+            mbar_init(&v_empty[i], 2);
         }
         for (int i = 0; i < kItemSlots; ++i) {
             mbar_init(&item_full[i], 1);
@@ -361,27 +347,23 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
         const uint32_t idesc_qk = make_idesc_bf16(128, kHalf, false, false);
         const int n_cols = kForm == kPadded ? (p.d_real + 15) & ~15 : D;  // columns of Q, K, V that are not all padding
         const uint32_t idesc_pv = make_idesc_bf16(128, n_cols, false, true);
-        const int tq = kSplit ? 0 : t;  // the Q tile
-        const uint32_t q_addr = smem_u32(sQ) + tq * Cfg::kTileBytes, k_addr = smem_u32(sK), v_addr = smem_u32(sV);
+        const uint32_t q_addr = smem_u32(sQ) + t * Cfg::kTileBytes, k_addr = smem_u32(sK), v_addr = smem_u32(sV);
         const uint32_t colS = tmem + (t ? Cfg::kColS1 : Cfg::kColS0), colO = tmem + (t ? Cfg::kColO1 : Cfg::kColO0);
         bool ok = true;
         // running counts over all items of this block (ring stages and barrier parities): key blocks of the rings,
         // key blocks and items of this tile
         uint32_t kb = 0, cb = 0, n_done = 0;
-        [[maybe_unused]] uint32_t n_q = 0;  // kSplit: loads of Q so far
         Item w;
         for (int it = 0; ok && fetch_item(it, w); ++it) {
             const uint32_t n_blk = t ? w.n_blk1 : w.n_blk0, n_max = w.n_max;
-            // place of this tile's (stream's) n-th key block in the rings
-            auto nth = [&](uint32_t n) -> uint32_t { return kb + (kSplit ? 2 * n + t : n); };
             if (n_blk > 0) {
-                ok = mbar_wait(&q_full[tq], (kSplit ? n_q : n_done) & 1, ctx, 20);
+                ok = mbar_wait(&q_full[t], n_done & 1, ctx, 20);
                 // S of half h of key block n: rows 64h.. of the block are the B operand (K-major panels, 64 rows = 8192
                 // bytes down).  It goes where P of the same half of the block before lives: that product must have completed.
                 auto issue_qk = [&](uint32_t n, uint32_t h) -> bool {
-                    const uint32_t st = nth(n) % Cfg::kStages;
+                    const uint32_t st = (kb + n) % Cfg::kStages;
                     if (cb + n > 0 && !mbar_wait(&pv_done[t * 2 + h], (cb + n - 1) & 1, ctx, 22)) return false;
-                    if (h == 0 && !mbar_wait(&k_full[st], (nth(n) / Cfg::kStages) & 1, ctx, 21)) return false;
+                    if (h == 0 && !mbar_wait(&k_full[st], ((kb + n) / Cfg::kStages) & 1, ctx, 21)) return false;
                     tc_fence_after_sync();
                     const uint32_t b0 = k_addr + st * Cfg::kTileBytes + h * (kHalf * 128);
                     auto step = [&](int kk) {
@@ -397,18 +379,18 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                     }
                     umma_commit_pred(leader, &s_full[t * 2 + h]);
                     if (h == 1) umma_commit_pred(leader, &k_empty[st]);
-                    if (kMore && h == 1 && n + 1 == n_blk) umma_commit_pred(leader, &q_empty[tq]);
+                    if (kMore && h == 1 && n + 1 == n_blk) umma_commit_pred(leader, &q_empty[t]);
                     if (t == 0) GQA_FTRACE(1, 2 * n + h, 0);
                     return true;
                 };
                 if (ok) ok = issue_qk(0, 0);
 #pragma unroll 1
                 for (uint32_t n = 0; n < n_blk && ok; ++n) {
-                    const uint32_t st = nth(n) % Cfg::kStages;
+                    const uint32_t st = (kb + n) % Cfg::kStages;
 #pragma unroll
                     for (uint32_t h = 0; h < 2; ++h) {
                         if (ok && (h == 0 || n + 1 < n_blk)) ok = issue_qk(n + h, h ^ 1);  // the next S
-                        if (ok && h == 0) ok = mbar_wait(&v_full[st], (nth(n) / Cfg::kStages) & 1, ctx, 23);
+                        if (ok && h == 0) ok = mbar_wait(&v_full[st], ((kb + n) / Cfg::kStages) & 1, ctx, 23);
                         if (ok && h == 0 && n == 0 && n_done > 0) ok = mbar_wait(&o_empty[t], (n_done - 1) & 1, ctx, 25);  // the item before has read O
                         if (ok) ok = mbar_wait(&p_full[t * 2 + h], (cb + n) & 1, ctx, 24);
                         if (!ok) break;
@@ -426,16 +408,10 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                     }
                 }
                 ++n_done;
-            } else if (kSplit && kMore && n_max > 0) {
-                // a tile of one key block: the second stream has no use for its Q (waited for, so that the arrival falls into
-                // the right phase)
-                ok = mbar_wait(&q_full[0], n_q & 1, ctx, 28);
-                if (ok && leader) mbar_arrive(&q_empty[0]);
             }
-            if (kSplit && n_max > 0) ++n_q;
             // blocks that only the other tile uses: released as soon as they are there (waited for, so that the arrival
             // falls into the right phase)
-            for (uint32_t n = n_blk; !kSplit && n < n_max && ok; ++n) {
+            for (uint32_t n = n_blk; n < n_max && ok; ++n) {
                 const uint32_t st = (kb + n) % Cfg::kStages;
                 const uint32_t par = ((kb + n) / Cfg::kStages) & 1;
                 ok = mbar_wait(&k_full[st], par, ctx, 26);
@@ -449,16 +425,14 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
         }
     } else {
         // ======================= softmax warpgroups =======================
-        const int t = warp >> 2;                      // query tile (kSplit: stream of the tile) owned by this warpgroup
-        constexpr int kTileRows = kSplit ? 0 : kTile; // from one warpgroup's query tile to the next one's
+        const int t = warp >> 2;                      // query tile owned by this warpgroup
         const int r = (warp & 3) * 32 + lane;         // row inside the tile == TMEM lane
-        [[maybe_unused]] uint32_t n_done_other = 0;   // kSplit: items of the other stream so far
         uint32_t cb = 0, n_done = 0;                  // key blocks and items of this tile so far (barrier parities)
         bool ok = true;
         Item w;
         for (int it = 0; ok && fetch_item(it, w); ++it) {
             const int n_blk = t ? w.n_blk1 : w.n_blk0;
-            if (kSplit ? w.n_max == 0 : n_blk == 0) {
+            if (n_blk == 0) {
                 if constexpr (kMore) continue;
                 else break;
             }
@@ -470,12 +444,11 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
             const float c = p.scale_log2;
             const uint64_t c2 = pack_f32x2(c, c);
             const int total = 2 * n_blk;
-            const int diag_block = (q0 + t * kTileRows) / kTile;  // only this block needs the causal mask
+            const int diag_block = (q0 + t * kTile) / kTile;  // only this block needs the causal mask
             float m_run = -INFINITY;  // running maximum of the raw logits that P is measured against
             float l_run = 0.f;
             for (int j = 0; j < total; ++j) {
                 const int n = j >> 1, h = j & 1;
-                const int kblk = kSplit ? 2 * n + t : n;  // key block of the sequence
                 ok = mbar_wait(&s_full[t * 2 + h], (cb + n) & 1, ctx, 30);
                 if (!ok) break;
                 tc_fence_after_sync();
@@ -483,8 +456,8 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                 if (warp == 4) GQA_FTRACE(2, j, 0);
                 if (t == 0) GQA_FTRACE(4, j, warp & 3);
                 // last valid column of this row inside the 128-key block: the causal diagonal and / or the end of S
-                const bool diag = p.causal && (kblk == diag_block);
-                const int s_left = len - kblk * kTile;  // keys of this block that exist
+                const bool diag = p.causal && (n == diag_block);
+                const int s_left = len - n * kTile;  // keys of this block that exist
                 const bool masked = diag || s_left < kTile;
                 const int lim = min(diag ? r : kTile - 1, s_left - 1);
                 const int col0 = h * kHalf;  // column of v[0] inside the 128-key block
@@ -585,58 +558,6 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                 if (warp == 4) GQA_FTRACE(2, j, 2);
                 GQA_FTRACE(t == 0 ? 3 : 5, j, warp & 3);
             }
-            if constexpr (kSplit) {
-                // epilogue: the two streams' O, each weighted with its share of the row sum; a warpgroup stores half of the columns
-                const int n_other = t ? w.n_blk0 : w.n_blk1;
-                if (ok && n_blk > 0) {
-                    ok = mbar_wait(&o_full[t], n_done & 1, ctx, 31);  // (and so the other warpgroup has read the item before's)
-                    ml[t * kTile + r] = make_float2(m_run, l_run);
-                    mbar_arrive(&merge_full[t]);
-                }
-                if (ok && n_other > 0)
-                    ok = mbar_wait(&merge_full[t ^ 1], n_done_other & 1, ctx, 33) && mbar_wait(&o_full[t ^ 1], n_done_other & 1, ctx, 34);
-                if (ok) {
-                    tc_fence_after_sync();
-                    const bool row_ok = q0 + r < len;
-                    const bool both = w.n_blk1 > 0;
-                    const float2 s0 = ml[r], s1 = both ? ml[kTile + r] : make_float2(-INFINITY, 0.f);
-                    const float m = fmaxf(s0.x, s1.x);
-                    const float e0 = ex2_approx((s0.x - m) * c), e1 = ex2_approx((s1.x - m) * c);
-                    const float l = s0.y * e0 + s1.y * e1;
-                    const float a0 = e0 / l, a1 = e1 / l;
-                    const size_t grow_ = (size_t)q_row0 + r;
-                    __nv_bfloat16* orow = p.bshd ? p.O + ((size_t)(b * p.S + y0 + q0 + r) * p.Hq + hq) * D : p.O + grow_ * p.d_real;
-                    const uint32_t tO0 = tmem + lane_addr + Cfg::kColO0, tO1 = tmem + lane_addr + Cfg::kColO1;
-#pragma unroll 1
-                    for (int col = t * (D / 2); col < (t + 1) * (D / 2) && col < p.d_real; col += 16) {
-                        uint32_t x[16], y[16];
-                        tmem_ld16(tO0 + col, x);
-                        if (both) tmem_ld16(tO1 + col, y);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int i = 0; i < 16; ++i)
-                            x[i] = __float_as_uint(__uint_as_float(x[i]) * a0 + (both ? __uint_as_float(y[i]) * a1 : 0.f));
-#pragma unroll
-                        for (int i = 0; i < 2; ++i) {
-                            uint4 o;
-                            o.x = pack_bf16x2(__uint_as_float(x[8 * i + 0]), __uint_as_float(x[8 * i + 1]));
-                            o.y = pack_bf16x2(__uint_as_float(x[8 * i + 2]), __uint_as_float(x[8 * i + 3]));
-                            o.z = pack_bf16x2(__uint_as_float(x[8 * i + 4]), __uint_as_float(x[8 * i + 5]));
-                            o.w = pack_bf16x2(__uint_as_float(x[8 * i + 6]), __uint_as_float(x[8 * i + 7]));
-                            if (row_ok && col + i * 8 < p.d_real) *reinterpret_cast<uint4*>(orow + col + i * 8) = o;
-                        }
-                    }
-                    if (t == 0 && p.LSE && row_ok) p.LSE[grow_] = (m * c + log2f(l)) * kLn2;
-                    tc_fence_before_sync();
-                    mbar_arrive(&o_empty[0]);
-                    if (both) mbar_arrive(&o_empty[1]);
-                }
-                if constexpr (!kMore) break;
-                cb += n_blk;
-                n_done += n_blk > 0;
-                n_done_other += n_other > 0;
-                continue;
-            }
             // epilogue: O / l -> bf16, LSE
             if (ok) ok = mbar_wait(&o_full[t], n_done & 1, ctx, 31);
             if (ok) {
@@ -683,28 +604,6 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     }
 }
 
-// Whether to launch one query tile per item with its key blocks in two streams (kSplit) or two tiles per item: the estimated
-// time of either, in steps of two (tile, key block) pairs, of `n1` items of one tile or `n2` of two.  The split halves the
-// longest chain and the grain of the work; its blocks load twice the K and V per step (D = 128 has room for two stages of the
-// rings only, one per stream) and finish twice as many items.  B200, Hq16, us, pairs against split: D = 64 S2048 causal
-// 30.6 / 21.6, S3072 43.1 / 38.3, S4096 55.3 / 56.2; not causal S512 9.0 / 7.8, S2560 67.1 / 53.2, S4096 103.8 / 103.0; D = 128
-// causal S1536 28.1 / 20.8, S3072 52.4 / 54.3, not causal S1024 15.7 / 14.3, S1536 30.3 / 36.3, S2560 75.6 / 80.5; B4 Hq32 S256
-// D64 causal 7.8 / 9.9; B1 Hq4 S8192 D64 causal 106.3 / 54.4.
-template <int D>
-bool split_pays(int n_tiles, long long n1, long long n2, bool causal, bool packed) {
-    const long long sms = sm_count();
-    if (n1 <= sms) return true;  // every tile finds an SM at once
-    if (packed || n1 > 4 * sms) return false;  // (the lengths are not known here; the rounds of long launches even out)
-    auto rounds = [&](long long n) { return (double)((n + sms - 1) / sms); };
-    const int half = (n_tiles + 1) / 2;
-    if (!causal) return rounds(n1) * (half * (D == 64 ? 1.0 : 1.45) + 1.0) < rounds(n2) * (n_tiles + 1.0);
-    // items of all lengths, longest first: the longest one or the average share of an SM sets the end
-    double steps = 0;  // of one head
-    for (int i = 1; i <= n_tiles; ++i) steps += (i + 1) / 2;
-    const double share = steps * (double)(n1 / n_tiles) / (double)sms;
-    return std::max((double)half, share) * (D == 64 ? 1.25 : 1.45) + rounds(n1) < std::max((double)n_tiles, share) + rounds(n2);
-}
-
 template <int D>
 int launch_fwd_t(const void* Q, const void* K, const void* V, void* O, float* LSE, const Shape& s, unsigned int* status,
                  cudaStream_t stream) {
@@ -731,8 +630,9 @@ int launch_fwd_t(const void* Q, const void* K, const void* V, void* O, float* LS
     p.bshd = s.bshd;
     p.d_real = s.D;
     p.cu = s.cu_seqlens;
-    // Two query tiles per item share the K/V blocks and keep the tensor core busy in turns; short launches take one tile per
-    // item (see split_pays).
+    // Two query tiles per item share the K/V blocks and keep the tensor core busy in turns; one tile per item finishes
+    // sooner when every tile gets an SM of its own.  B200, D = 128 causal: 128 tiles (B1 Hq16 S1024) 22.5 us as single
+    // tiles against 25.6 us as pairs; 192 tiles (B2 Hq12 S1000) 30.8 against 26.6: the second round costs more.
     const int n_tiles = ((s.cu_seqlens ? s.max_seqlen : s.S) + kTile - 1) / kTile, n_seqs = s.cu_seqlens ? s.n_seqs : s.B;
     // Items of a packed batch are listed where there are not too many sequences; every sequence ends with one partial item at
     // the most, which bounds the list.
@@ -741,28 +641,26 @@ int launch_fwd_t(const void* Q, const void* K, const void* V, void* O, float* LS
         const long long all = (long long)((n_tiles + tiles - 1) / tiles) * n_seqs;
         return s.Hq * (p.n_listed ? std::min(all, (long long)s.S / (tiles * kTile) + n_seqs) : all);
     };
-    const bool split = n_tiles > 1 && split_pays<D>(n_tiles, items(1), items(2), s.causal, s.cu_seqlens != nullptr);
-    p.tiles = split || items(1) <= sm_count() ? 1 : 2;
+    p.tiles = items(1) <= sm_count() ? 1 : 2;
     p.n_groups = (n_tiles + p.tiles - 1) / p.tiles;
     p.scale_log2 = s.scale * kLog2e;
     // Causal items are of very different length: the longest of all heads first keeps the end of the launch short, as long as
     // L2 holds K and V of what runs at a time (head by head they are read from memory once, however long the launch).  B200, us:
     // B1 Hq16 S4096 D128 94.0 -> 65.0, D64 82.2 -> 55.3; B1 Hq32 S2048 D128 71.9 -> 51.5; B16 Hq16 Hkv2 S4096 D64 (34 MB of K and
     // V) 764 -> 737, but B8 Hq32 Hkv8 S8192 D128 (268 MB) 3 968 -> 4 130.
-    p.tile_slow = s.causal && !s.cu_seqlens && (split || s.kv_rows() * s.D * 4 <= kOrderKvBytes);
+    p.tile_slow = s.causal && !s.cu_seqlens && s.kv_rows() * s.D * 4 <= kOrderKvBytes;
     const dim3 grid = p.n_listed    ? dim3((unsigned)items(p.tiles))
                       : p.tile_slow ? dim3(s.Hq, n_seqs, p.n_groups)
                                     : dim3(p.n_groups, s.Hq, n_seqs);
     const bool more = items(p.tiles) > sm_count();
     auto pick = [&](auto form) {
         constexpr Form F = decltype(form)::value;
-        return split ? (more ? gqa_fwd_sm100_kernel<D, F, true, true> : gqa_fwd_sm100_kernel<D, F, false, true>)
-                     : (more ? gqa_fwd_sm100_kernel<D, F, true, false> : gqa_fwd_sm100_kernel<D, F, false, false>);
+        return more ? gqa_fwd_sm100_kernel<D, F, true> : gqa_fwd_sm100_kernel<D, F, false>;
     };
     auto kernel = s.cu_seqlens ? pick(std::integral_constant<Form, kPacked>{})
                   : s.D != D   ? pick(std::integral_constant<Form, kPadded>{})
                                : pick(std::integral_constant<Form, kNative>{});
-    const int smem = s.cu_seqlens ? Cfg::kOffList + (int)sizeof(PackedList) : split ? Cfg::kOffList : Cfg::kSmemTotal;
+    const int smem = Cfg::kSmemTotal + (s.cu_seqlens ? (int)sizeof(PackedList) : 0);
     GQA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     GQA_CUDA_TRY(launch_after(kernel, grid, kFwdThreads, smem, stream, mq, mk, mv, p));
     count_launch();

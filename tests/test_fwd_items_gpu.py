@@ -33,11 +33,11 @@ BATCHED = [
     (1, 4, 2, 4731, 64),     # 148 tiles: one tile per item
     (1, 4, 2, 4737, 128),    # 152 tiles: two per item, the last one of a head holds one row
     (5, 6, 2, 640, 40),      # 150 tiles, head dimension below the kernel's
-    (1, 16, 4, 1280, 64),    # 160 tiles, two streams of key blocks per tile (causal: tiles of one block among them)
-    (1, 16, 4, 1537, 128),   # 208 tiles, two streams when causal; the last tile of a head holds one row
-    (4, 32, 8, 256, 64),     # 256 tiles of one and two key blocks: pairs
+    (1, 16, 4, 1280, 64),    # 160 tiles in 80 pairs
+    (1, 16, 4, 1537, 128),   # 208 tiles; the last tile of a head holds one row
+    (4, 32, 8, 256, 64),     # 256 tiles of one and two key blocks
     (2, 24, 8, 129, 128),    # 96 tiles, the second key block holds one key
-    (1, 16, 4, 2560, 64),    # 320 tiles, two streams over several rounds
+    (1, 16, 4, 2560, 64),    # 160 pairs: more items than SMs by a few
 ]
 
 
@@ -56,6 +56,30 @@ def test_items_batched(gqa_lib, shape, causal):
         for g in range(Hkv):
             h = slice(g * G, (g + 1) * G)
             _check(o[b, h], lse[b, h], q[b, h], k[b, g], v[b, g], scale, causal)
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("Hq,Hkv,S,D", [
+    (4, 2, 640, 64),
+    (12, 4, 1000, 128),
+    (6, 2, 256, 64),
+    (16, 4, 1024, 80),
+    (2, 2, 3000, 128),
+])
+def test_bits_do_not_depend_on_the_launch(gqa_lib, Hq, Hkv, S, D, causal):
+    """O and LSE of a sequence are the same bits alone (one tile per item), among a few and in a large batch (pairs, several
+    items per SM), and of a head's shard alone: a row's arithmetic depends on its own tile and nothing else."""
+    B = 24
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    q, k, v = (torch.randn(B, h, S, D, generator=gen, device="cuda").bfloat16() for h in (Hq, Hkv, Hkv))
+    o, lse = ops.gqa_forward(q, k, v, causal=causal)
+    for n in (1, 2, 5):
+        o_n, lse_n = ops.gqa_forward(q[:n], k[:n], v[:n], causal=causal)
+        assert torch.equal(o_n, o[:n]) and torch.equal(lse_n, lse[:n]), n
+    G = Hq // Hkv
+    o_1, lse_1 = ops.gqa_forward(q[:1, :G].contiguous(), k[:1, :1].contiguous(), v[:1, :1].contiguous(), causal=causal)
+    assert torch.equal(o_1, o[:1, :G]) and torch.equal(lse_1, lse[:1, :G])
+    ops.check_status()
 
 
 @pytest.mark.parametrize("causal", [False, True])
