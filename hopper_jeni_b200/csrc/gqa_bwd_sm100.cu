@@ -188,7 +188,7 @@ struct BwdParams {
     const int* cu;  // packed variable-length batch: sequence starts (n_seqs + 1), else null
     int n_seqs, run;  // packed batch: sequences, and how many of them form a super-group of the work list (0 = no list)
     int sg;       // causal order: (batch, KV head) groups per super-group (see the work-item comment)
-    int lead;     // deterministic causal order: KV tiles at the head of the list that come in descending order (same comment)
+    int lead;     // deterministic causal order: KV tiles at the head of a group that come in descending order (same comment)
     int n_items;  // n_tiles * groups * parts: work items, each handled by one thread block at a time
     int Hq, Hkv, S, causal, n_tiles, G, bshd;
     int d_real;  // head dimension of the tensors (<= D of the kernel; the columns beyond it read as zeros)
@@ -283,10 +283,14 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     // must reduce one after the other, and this order keeps only a few of them in flight together.  It is launched
     // with one block per item: its blocks wait for one another, and a block that waits must never hold the SM that
     // the block it waits for needs (blocks are dispatched in index order, and a block only waits for lower ones).
-    // Its causal list begins with the KV tiles that find an SM at once (`lead` of every group) in descending order: all
-    // of them start together, tile kt on query tile kt, so kt + 1 is one query tile ahead of kt and nobody waits.  In
-    // ascending order block kt + 1 had to follow block kt, although it has fewer query tiles, and took as long.
-    // B200, B2 Hq24 Hkv8 S4096 D128: 840 -> 790 us; B1 Hq64 Hkv8 S11840 D64, forward and backward: 6 645 -> 6 453 us.
+    // Its causal list begins with the first `lead` KV tiles of every group in descending order: those that start together,
+    // tile kt on query tile kt, find kt + 1 one query tile ahead of kt, and nobody waits.  In ascending order block kt + 1 has to
+    // follow block kt, although it has fewer query tiles, and takes as long.  The order is that of the fp32 sums, so `lead`
+    // depends on S alone: dQ of a sequence is the same bits in any batch, on any shard and on a chip with any number of SMs.
+    // B200, us, lead 0 / 4 / 8: B2 Hq24 Hkv8 S4096 D128 846 / 816 / 763, B16 Hq16 Hkv2 S2048 D64 763 / 711 / 686, B2 Hq8 Hkv8
+    // S1024 D128 72 / 63 / 50; but with more groups, where fewer tiles of one start together, B8 Hq32 Hkv8 S4096 D128
+    // 4 487 / 4 423 / 4 578, B4 Hq32 Hkv8 S1024 D128 227 / 192 / 224, B16 Hq32 Hkv8 S1024 D128 767 / 790 / 830: 4 costs 3 % at
+    // the most.  (As many as find an SM at once, which makes the bits depend on the launch: 746, 708, 50; 4 348, 192, 768.)
     struct WorkItem {
         int kt, grp, part, b, hkv, qt0, n_qt, n_iter, kv_x, kv_z;
         int shift;  // the item's loop over the query tiles of a head starts at tile qt0 + shift and wraps around
@@ -1116,6 +1120,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
 // The bound keeps the end of the launch balanced: a super-group must last about as long as its longest item
 // (n_tiles tile pairs per head against sg * n_tiles * (n_tiles + 1) / 2 spread over the SMs), or the long items of
 // the last super-group would start too late for the others to level them out.
+constexpr int kOrderedLead = 4;  // see the work-item comment
 int super_group_bound(int n_tiles, int sms) { return (2 * sms + n_tiles) / (n_tiles + 1); }  // ceil(2 * sms / (n_tiles + 1))
 int causal_super_group(int groups, int n_tiles, int sms) {
     const int bound = super_group_bound(n_tiles, sms);
@@ -1189,7 +1194,7 @@ int launch_bwd_t(const void* Q, const void* K, const void* V, const void* dO, co
         p.run = s.causal ? std::min((super_group_bound(p.n_tiles, sm_count()) + s.Hkv - 1) / s.Hkv, s.n_seqs) : 1;
     p.sg = dq_turn ? p.groups : causal_super_group(p.groups, p.n_tiles, sm_count());
     p.n_items = p.n_tiles * p.groups * parts;
-    p.lead = dq_turn && s.causal ? std::min(p.n_tiles, sm_count() / (p.groups * parts)) : 0;
+    p.lead = dq_turn && s.causal ? std::min(p.n_tiles, kOrderedLead) : 0;
     // persistent, one block per SM (shared memory and TMEM allow no second), except in the deterministic mode (see the
     // work-item comment in the kernel)
     const unsigned grid = (unsigned)(dq_turn ? p.n_items : std::min(p.n_items, sm_count()));

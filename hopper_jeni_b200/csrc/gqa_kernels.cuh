@@ -70,8 +70,8 @@ int launch_fwd_sm100(const void* Q, const void* K, const void* V, void* O, float
                      unsigned int* status, cudaStream_t stream);
 // Stage 2 of the backward: KV-tile-parallel main kernel (tcgen05 + TMEM + TMA); dK/dV written
 // once per element, dQ accumulated into dq_accum with fp32 reductions.
-// With dq_turn (zeroed counters, one per 32 query rows) the reductions of every dQ tile are applied in KV-tile
-// order, which makes dQ bit-reproducible; nullptr = unordered.  dq_accum == nullptr launches the variant without the
+// With dq_turn (zeroed counters, one per 32 query rows) the reductions of every dQ tile are applied in an order of the
+// KV tiles that S and the mask fix, which makes dQ bit-reproducible; nullptr = unordered.  dq_accum == nullptr launches the variant without the
 // dQ part (dK and dV only), for use with launch_bwd_dq_sm100.
 // With parts > 1 (a divisor of G) every KV tile is handled by `parts` thread blocks over disjoint query heads; their
 // fp32 dK / dV sums go to `partial` (BwdWorkspace::partial_bytes) and launch_dkdv_reduce adds them in a fixed order.

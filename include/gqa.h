@@ -98,8 +98,9 @@ int gqa_bwd(const void* Q, const void* K, const void* V, const void* O, const vo
 /*
  * gqa_bwd with option flags.  flags = 0 is gqa_bwd.
  * GQA_BWD_DETERMINISTIC: the fp32 reductions into every 32-row slice of the dQ accumulator are applied in
- * a fixed order of the KV tiles (a counter per slice in the workspace hands the turn from one thread block to the next), so dQ
- * is bit-reproducible from run to run as dK and dV always are.  The reference's dQ path is order-dependent
+ * an order of the KV tiles that S and the mask alone fix (a counter per slice in the workspace hands the turn from one thread
+ * block to the next), so dQ of a sequence is bit-reproducible from run to run, as dK and dV always are, and the same bits in any
+ * batch, in a shard of the groups and on any GPU.  The reference's dQ path is order-dependent
  * (cp.reduce.async.bulk add, src/attention/GQA_bwd_baseline.cu:360-365, run-to-run differences noted in
  * docs/report.md:115-116) and has no such switch; its determinism probe
  * (precision/vj1d_determinism_probe.cu:33) is what this mode is checked with.  Slower than the default

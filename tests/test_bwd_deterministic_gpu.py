@@ -70,14 +70,14 @@ def test_deterministic_backward_is_bit_reproducible(gqa_lib, shape, causal):
 
 
 @pytest.mark.parametrize("shape", [
-    (1, 2, 1, 1664, 64),     # one group: every KV tile finds an SM, all of them in descending order
-    (2, 40, 20, 1024, 128),  # 40 groups: the first three of eight KV tiles
-    (1, 74, 74, 700, 64),    # two of six, a partial last tile
-    (10, 16, 16, 300, 64),   # more groups than SMs: none
-    (1, 4, 2, 520, 72),      # a head dimension that is not native
+    (1, 2, 1, 1664, 64),     # one group of 13 KV tiles
+    (2, 40, 20, 1024, 128),  # 40 groups of eight
+    (1, 74, 74, 700, 64),    # 74 groups of six, a partial last tile
+    (10, 16, 16, 300, 64),   # more groups than SMs, fewer tiles than come in descending order
+    (1, 4, 2, 520, 72),      # one tile more than those; a head dimension that is not native
 ])
 def test_causal_order_of_the_reductions(gqa_lib, shape):
-    """The causal list starts with the KV tiles that find an SM at once, in descending order, and the turns follow it.  Three
+    """The causal list starts with the first four KV tiles of a group in descending order, and the turns follow it.  Three
     runs bit-identical, dK and dV the default mode's bits, dQ its sums in another order (as above)."""
     B, Hq, Hkv, S, D = shape
     gen = torch.Generator(device="cuda").manual_seed(6)
@@ -96,6 +96,27 @@ def test_causal_order_of_the_reductions(gqa_lib, shape):
     assert torch.equal(runs[0][1], want[1]) and torch.equal(runs[0][2], want[2])
     m = util.metrics(util.to_np(runs[0][0]), util.to_np(want[0]))
     assert m["rel_rms"] < 2e-3, m
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("Hq,Hkv,S,D", [(4, 2, 640, 64), (4, 4, 300, 64), (6, 2, 1100, 128), (4, 2, 2048, 80)])
+def test_ordered_gradients_do_not_depend_on_the_launch(gqa_lib, Hq, Hkv, S, D, causal):
+    """The order of the fp32 sums depends on S and the mask alone: the gradients of a sequence are the same bits alone, in
+    batches of every size and on a shard that holds one KV head."""
+    B, G = 40, Hq // Hkv
+    gen = torch.Generator(device="cuda").manual_seed(12)
+    q, do = (torch.randn(B, Hq, S, D, generator=gen, device="cuda").bfloat16() for _ in range(2))
+    k, v = (torch.randn(B, Hkv, S, D, generator=gen, device="cuda").bfloat16() for _ in range(2))
+    o, lse = ops.gqa_forward(q, k, v, causal=causal)
+
+    def grads(n, hq=Hq, hkv=Hkv):
+        args = [t[:n, :h].contiguous() for t, h in ((q, hq), (k, hkv), (v, hkv), (o, hq), (do, hq), (lse, hq))]
+        return ops.gqa_backward(*args, causal=causal, deterministic=True)
+
+    whole = grads(B)
+    for n, hq, hkv in ((1, Hq, Hkv), (7, Hq, Hkv), (1, G, 1)):
+        for got, want, h in zip(grads(n, hq, hkv), whole, (hq, hkv, hkv)):
+            assert torch.equal(got, want[:n, :h]), (n, hq)
 
 
 def test_unknown_flag_bits_are_refused(gqa_lib):
