@@ -235,13 +235,16 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
         mbar_init(clc_full, 1);
         fence_mbar_init();
     }
+    // Everything above overlaps the end of the kernel in front in the stream; global memory is first used from here on.  Tensor
+    // memory is taken after the wait as well: held before it, a kernel in front that lets its dependents come up before it has
+    // taken its own would wait for this block, and this block for the end of that kernel.
+    // It pays for forwards back to back only.  B200: B1 Hq4 S128 D64 5.75 -> 4.8 us, on inputs from memory 6.3 -> 5.1; B2 Hq12 S1000
+    // D128 19.8 -> 19.1; behind a cuBLAS product or an element-wise kernel no gain (8.0 -> 8.0 and 23.8 -> 24.1 with that kernel).
+    pdl_wait();
     if (warp == kWarpMma0) {
         tmem_alloc(tmem_slot, Cfg::kTmemCols);
         tmem_relinquish();
     }
-    // Everything above overlaps the end of the kernel in front in the stream; global memory is first used from here on.
-    // B200, calls back to back: B1 Hq4 S128 D64 7.3 -> 6.3 us, B2 Hq12 S1000 D128 21.4 -> 19.4 us.
-    pdl_wait();
     // a non-zero status word (a bounded wait gave up earlier and nobody has read the report yet) makes
     // every later thread block skip its work, so a wedged launch drains in one wave
     if (tid == 0) *abort_flag = (*reinterpret_cast<volatile unsigned int*>(p.status) != 0u) ? 98u : 0u;

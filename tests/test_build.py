@@ -1,5 +1,5 @@
 """CPU tests of the build rules: the C libraries and the harness need nvcc only, and the torch binding is built anew for
-another torch or interpreter."""
+another torch or interpreter; and of one rule of the sources that no run can show."""
 import os
 import subprocess
 
@@ -20,3 +20,11 @@ def test_default_target_needs_no_python_and_no_torch():
 def test_binding_is_rebuilt_for_another_abi():
     assert "torch_binding.cpp" not in _dry_run("binding").stdout  # built, up to date
     assert "torch_binding.cpp" in _dry_run("binding", "BINDING_ABI=another-torch-or-interpreter").stdout
+
+
+def test_forward_takes_tensor_memory_behind_its_wait():
+    """The forward may come up under the end of any kernel, also of one that has let it start before taking its own tensor
+    memory: holding some while it waits for that kernel's end, it could keep it from ever ending."""
+    with open(os.path.join(CSRC, "gqa_fwd_sm100.cu")) as f:
+        src = f.read()
+    assert 0 < src.rindex("pdl_wait();") < src.index("tmem_alloc(")
