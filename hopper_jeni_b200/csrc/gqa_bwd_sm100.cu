@@ -168,7 +168,7 @@ struct BwdCfg {
     static constexpr uint32_t kColP = (D == 64) ? 448 : 0;
     static_assert(kColDK + D + (kPAliasesS ? 0 : 64) <= 512, "TMEM budget");
     static constexpr int kOffList = kSmemTotal;  // packed batches: the work list
-    static_assert(kSmemTotal + (int)sizeof(PackedList) <= 227 * 1024, "shared memory budget");
+    static_assert(kOffList % alignof(PackedList) == 0 && kSmemTotal + (int)sizeof(PackedList) <= 227 * 1024, "shared memory budget");
     static_assert(kSmemTotal > 114 * 1024, "one CTA per SM is assumed by the 512-column TMEM allocation");
 };
 
@@ -1190,8 +1190,11 @@ int launch_bwd_t(const void* Q, const void* K, const void* V, const void* dO, co
     p.groups = (varlen ? s.n_seqs : s.B) * s.Hkv;
     p.n_seqs = s.n_seqs;
     p.run = 0;
-    if (varlen && s.n_seqs <= kMaxListedSeqs)
+    if (varlen && list_pays(s.n_seqs, s.max_seqlen, s.S, kTile, s.Hkv, sm_count())) {
         p.run = s.causal ? std::min((super_group_bound(p.n_tiles, sm_count()) + s.Hkv - 1) / s.Hkv, s.n_seqs) : 1;
+        const bool one_run = !s.causal || p.run == s.n_seqs;  // super-groups of equal lengths: 32 of 300, Hq16 D128 145 -> 137 us
+        if (one_run && !lengths_differ(s.n_seqs, s.max_seqlen, s.S)) p.run = 0;
+    }
     p.sg = dq_turn ? p.groups : causal_super_group(p.groups, p.n_tiles, sm_count());
     p.n_items = p.n_tiles * p.groups * parts;
     p.lead = dq_turn && s.causal ? std::min(p.n_tiles, kOrderedLead) : 0;

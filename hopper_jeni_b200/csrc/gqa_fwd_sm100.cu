@@ -70,7 +70,7 @@ struct FwdCfg {
     static constexpr uint32_t kTmemCols = 512;
     static constexpr uint32_t kColS0 = 0, kColS1 = 128, kColO0 = 256, kColO1 = 256 + D;
     static_assert(256 + 2 * D <= 512, "TMEM budget");
-    static_assert(kSmemTotal + (int)sizeof(PackedList) <= 227 * 1024, "shared memory budget");
+    static_assert(kOffList % alignof(PackedList) == 0 && kSmemTotal + (int)sizeof(PackedList) <= 227 * 1024, "shared memory budget");
     static_assert(kSmemTotal > 114 * 1024, "one CTA per SM is assumed by the 512-column TMEM allocation");
 };
 
@@ -129,7 +129,7 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     uint8_t* clc_answer = reinterpret_cast<uint8_t*>(clc_full + 2);
     constexpr int kBars = 16 + 4 * Cfg::kStages + 4 + 2 * kItemSlots + 2;
     static_assert(kBars % 2 == 0, "the answer is 16-byte aligned");
-    volatile int* item_slot = reinterpret_cast<volatile int*>(clc_answer + 16);  // [kItemSlots][4]: x, y, z of the block
+    volatile int* item_slot = reinterpret_cast<volatile int*>(clc_answer + 16);  // [kItemSlots][4]: x, y, z of the block (packed: hq, q0, y0, len)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(clc_answer + 16 + kItemSlots * 16);
     volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(tmem_slot + 1);
     static_assert(kBars * 8 + 16 + kItemSlots * 16 + 8 <= Cfg::kBarBytes, "barrier area");
@@ -154,37 +154,17 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     };
     // Packed variable-length batch: the sequence is a row range [y0, y0 + len) of the one [T, H*D] matrix; rows past
     // its end belong to the next sequence (or read as zeros past T): as keys they are masked like keys beyond S,
-    // as queries they are computed and not stored.  The grid covers max_seqlen: an item beyond its sequence has
-    // n_tiles = 0 and no key blocks; the producer passes most of them over, and every role does nothing in one.
-    PackedList* list = reinterpret_cast<PackedList*>(smem + Cfg::kOffList);
-    auto decode = [&](int x, int y, int z) -> Item {
+    // as queries they are computed and not stored.  An item beyond its sequence (the grid covers max_seqlen) or beyond the
+    // end of the work list has n_tiles = 0 and no key blocks; the producer passes most of them over, and every role does
+    // nothing in one.
+    [[maybe_unused]] PackedList* list = reinterpret_cast<PackedList*>(smem + Cfg::kOffList);
+    auto item_at = [&](int hq, int q0, int b, int y0, int len) -> Item {
         Item w;
-        int n_groups = p.n_groups;
-        if (kForm == kPacked && p.n_listed > 0) {  // the longest sequence first, head by head
-            const int u = list->run_of(x, p.n_listed);
-            const int r = x - list->first[u];
-            n_groups = (list->first[u + 1] - list->first[u]) / p.Hq;
-            if (r >= n_groups * p.Hq) return Item{};  // beyond the end of the list
-            z = list->seq[u];
-            y = r / n_groups;
-            x = r % n_groups;
-        } else if (p.tile_slow) {
-            const int place = z;
-            z = y;
-            y = x;
-            x = place;
-        }
-        const int idx = p.causal ? (n_groups - 1 - x) : x;  // heavy causal tiles first
-        w.hq = y;
-        w.q0 = idx * p.tiles * kTile;
-        w.b = z;
-        w.y0 = 0;
-        w.len = p.S;
-        if constexpr (kForm == kPacked) {
-            w.y0 = p.cu[z];
-            w.len = p.cu[z + 1] - w.y0;
-            w.b = 0;
-        }
+        w.hq = hq;
+        w.q0 = q0;
+        w.b = b;
+        w.y0 = y0;
+        w.len = len;
         w.n_tiles = w.q0 >= w.len ? 0 : (p.tiles == 2 && w.q0 + kTile < w.len) ? 2 : 1;
         const int n_blocks_all = (w.len + kTile - 1) / kTile;  // the last block may be partial: keys at and beyond len are masked
         w.n_blk0 = (w.n_tiles == 0) ? 0 : p.causal ? (w.q0 / kTile + 1) : n_blocks_all;
@@ -192,8 +172,37 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
         w.n_max = max(w.n_blk0, w.n_blk1);
         return w;
     };
+    auto decode = [&](int x, int y, int z) -> Item {
+        int n_groups = p.n_groups;
+        if constexpr (kForm == kPacked) {
+            if (p.n_listed > 0) {  // the longest sequence first, head by head
+                const int u = list->run_of(x, p.n_listed);
+                const int r = x - list->first[u];
+                n_groups = (list->first[u + 1] - list->first[u]) / p.Hq;
+                if (r >= n_groups * p.Hq) return Item{};  // beyond the end of the list
+                z = list->seq[u];
+                y = r / n_groups;
+                x = r % n_groups;
+            }
+        } else if (p.tile_slow) {
+            const int place = z;
+            z = y;
+            y = x;
+            x = place;
+        }
+        const int q0 = (p.causal ? (n_groups - 1 - x) : x) * p.tiles * kTile;  // heavy causal tiles first
+        if constexpr (kForm == kPacked) {
+            const int y0 = p.cu[z];
+            return item_at(y, q0, 0, y0, p.cu[z + 1] - y0);
+        } else {
+            return item_at(y, q0, z, 0, p.S);
+        }
+    };
     // The j-th item of this block, published by the producer; false = no more (or give up).  In the plain form every role
     // knows the only one.  (Knowing the first one here as well, with no wait for it: 389 against 382 us at B16 Hq16 S2048.)
+    // Of a packed batch the producer publishes the item itself: with every role looking the place up for itself (a search, two
+    // divisions and the sequence's limits from memory) short items are slower: B200, Hq16 Hkv4 D128 causal, 128 sequences of
+    // 300 tokens 208 us against 178, 600 of 1 to 200 tokens 290 against 268.
     auto fetch_item = [&](int j, Item& w) -> bool {
         int x = blockIdx.x, y = blockIdx.y, z = blockIdx.z;
         if constexpr (kMore) {
@@ -202,8 +211,13 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
             x = item_slot[sl * 4 + 0];
             y = item_slot[sl * 4 + 1];
             z = item_slot[sl * 4 + 2];
+            [[maybe_unused]] const int len = kForm == kPacked ? item_slot[sl * 4 + 3] : 0;
             mbar_arrive(&item_empty[sl]);
             if (x < 0) return false;
+            if constexpr (kForm == kPacked) {
+                w = item_at(x, y, 0, z, len);
+                return true;
+            }
         }
         w = decode(x, y, z);
         return true;
@@ -269,6 +283,7 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
             tma_prefetch_desc(&mapV);
             uint32_t n_claims = 0;
             int x = blockIdx.x, y = blockIdx.y, z = blockIdx.z;
+            [[maybe_unused]] Item next;  // packed batch: the item there
             // The next item: x = -1 when there is none.  False: a wait gave up.  Empty items of a packed batch are passed
             // over here, at 0.3 to 0.4 us each, while the other roles wait for the next one.  Long runs of them (a batch with many
             // empty sequences beside a long one) would outlast that wait, so every kMaxPassedOver-th is published: the
@@ -285,11 +300,16 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                         x = -1;
                         return true;
                     }
-                    if (kForm != kPacked || passed_over >= kMaxPassedOver || decode(x, y, z).n_tiles > 0) return true;
+                    if constexpr (kForm != kPacked) return true;
+                    next = decode(x, y, z);
+                    if (passed_over >= kMaxPassedOver || next.n_tiles > 0) return true;
                 }
             };
             bool ok = true;
-            if (kMore && kForm == kPacked && decode(x, y, z).n_tiles == 0) ok = claim();
+            if constexpr (kMore && kForm == kPacked) {
+                next = decode(x, y, z);
+                if (next.n_tiles == 0) ok = claim();
+            }
             uint32_t kb = 0;             // key blocks loaded so far, over all items
             int n_q[2] = {0, 0};         // loads of the two Q tiles so far
             for (int j = 0; ok; ++j) {
@@ -301,16 +321,23 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                         *abort_flag = 98u;
                         break;
                     }
-                    item_slot[sl * 4 + 0] = x;
-                    item_slot[sl * 4 + 1] = y;
-                    item_slot[sl * 4 + 2] = z;
+                    if constexpr (kForm == kPacked) {
+                        item_slot[sl * 4 + 0] = x < 0 ? -1 : next.hq;
+                        item_slot[sl * 4 + 1] = next.q0;
+                        item_slot[sl * 4 + 2] = next.y0;
+                        item_slot[sl * 4 + 3] = next.len;
+                    } else {
+                        item_slot[sl * 4 + 0] = x;
+                        item_slot[sl * 4 + 1] = y;
+                        item_slot[sl * 4 + 2] = z;
+                    }
                     mbar_arrive(&item_full[sl]);
                     if (x < 0) {
                         pdl_launch_dependents();
                         break;
                     }
                 }
-                const Item w = decode(x, y, z);
+                const Item w = kMore && kForm == kPacked ? next : decode(x, y, z);
                 const int hkv = w.hq / (p.Hq / p.Hkv);
                 // Tensor-map coordinates (x = column, y = position in the sequence, z = matrix).  [B,H,S,D] is B*H matrices
                 // [S, D]; [B,S,H,D] is B matrices [S, H*D] with the head at x = head * D.  Rows at y >= S read as zeros.
@@ -637,9 +664,12 @@ int launch_fwd_t(const void* Q, const void* K, const void* V, void* O, float* LS
     // sooner when every tile gets an SM of its own.  B200, D = 128 causal: 128 tiles (B1 Hq16 S1024) 22.5 us as single
     // tiles against 25.6 us as pairs; 192 tiles (B2 Hq12 S1000) 30.8 against 26.6: the second round costs more.
     const int n_tiles = ((s.cu_seqlens ? s.max_seqlen : s.S) + kTile - 1) / kTile, n_seqs = s.cu_seqlens ? s.n_seqs : s.B;
-    // Items of a packed batch are listed where there are not too many sequences; every sequence ends with one partial item at
+    // Items of a packed batch are listed where that pays and the lengths differ (equal ones are in order as they are: with the
+    // list 8 sequences of 300 tokens, Hq16 D128, take 18.4 us instead of 17.3).  Every sequence ends with one partial item at
     // the most, which bounds the list.
-    p.n_listed = s.cu_seqlens && n_seqs <= kMaxListedSeqs ? n_seqs : 0;
+    const bool listed = s.cu_seqlens && lengths_differ(n_seqs, s.max_seqlen, s.S) &&
+                        list_pays(n_seqs, s.max_seqlen, s.S, 2 * kTile, s.Hq, sm_count());
+    p.n_listed = listed ? n_seqs : 0;
     auto items = [&](int tiles) -> long long {
         const long long all = (long long)((n_tiles + tiles - 1) / tiles) * n_seqs;
         return s.Hq * (p.n_listed ? std::min(all, (long long)s.S / (tiles * kTile) + n_seqs) : all);
