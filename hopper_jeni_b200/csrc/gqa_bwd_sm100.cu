@@ -289,7 +289,8 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     // depends on S alone: dQ of a sequence is the same bits in any batch, on any shard and on a chip with any number of SMs.
     // B200, us, lead 0 / 4 / 8: B2 Hq24 Hkv8 S4096 D128 846 / 816 / 763, B16 Hq16 Hkv2 S2048 D64 763 / 711 / 686, B2 Hq8 Hkv8
     // S1024 D128 72 / 63 / 50; but with more groups, where fewer tiles of one start together, B8 Hq32 Hkv8 S4096 D128
-    // 4 487 / 4 423 / 4 578, B4 Hq32 Hkv8 S1024 D128 227 / 192 / 224, B16 Hq32 Hkv8 S1024 D128 767 / 790 / 830: 4 costs 3 % at
+    // 4 487 / 4 423 / 4 578, B4 Hq32 Hkv8 S1024 D128 227 / 192 / 224, B16 Hq32 Hkv8 S1024 D128 767 / 790 / 830.  Of a few tiles
+    // half (lead 0 / half / all): B14 Hkv8 S283 D64 174.5 / 176.6 / 180.9, B16 Hkv4 S384 D64 56.1 / 50.2 / 58.0.  It costs 2 to 3 % at
     // the most.  (As many as find an SM at once, which makes the bits depend on the launch: 746, 708, 50; 4 348, 192, 768.)
     struct WorkItem {
         int kt, grp, part, b, hkv, qt0, n_qt, n_iter, kv_x, kv_z;
@@ -1120,7 +1121,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
 // The bound keeps the end of the launch balanced: a super-group must last about as long as its longest item
 // (n_tiles tile pairs per head against sg * n_tiles * (n_tiles + 1) / 2 spread over the SMs), or the long items of
 // the last super-group would start too late for the others to level them out.
-constexpr int kOrderedLead = 4;  // see the work-item comment
+int ordered_lead(int n_tiles) { return std::min((n_tiles + 1) / 2, 4); }  // see the work-item comment
 int super_group_bound(int n_tiles, int sms) { return (2 * sms + n_tiles) / (n_tiles + 1); }  // ceil(2 * sms / (n_tiles + 1))
 int causal_super_group(int groups, int n_tiles, int sms) {
     const int bound = super_group_bound(n_tiles, sms);
@@ -1197,7 +1198,7 @@ int launch_bwd_t(const void* Q, const void* K, const void* V, const void* dO, co
     }
     p.sg = dq_turn ? p.groups : causal_super_group(p.groups, p.n_tiles, sm_count());
     p.n_items = p.n_tiles * p.groups * parts;
-    p.lead = dq_turn && s.causal ? std::min(p.n_tiles, kOrderedLead) : 0;
+    p.lead = dq_turn && s.causal ? ordered_lead(p.n_tiles) : 0;
     // persistent, one block per SM (shared memory and TMEM allow no second), except in the deterministic mode (see the
     // work-item comment in the kernel)
     const unsigned grid = (unsigned)(dq_turn ? p.n_items : std::min(p.n_items, sm_count()));

@@ -73,11 +73,11 @@ def test_deterministic_backward_is_bit_reproducible(gqa_lib, shape, causal):
     (1, 2, 1, 1664, 64),     # one group of 13 KV tiles
     (2, 40, 20, 1024, 128),  # 40 groups of eight
     (1, 74, 74, 700, 64),    # 74 groups of six, a partial last tile
-    (10, 16, 16, 300, 64),   # more groups than SMs, fewer tiles than come in descending order
-    (1, 4, 2, 520, 72),      # one tile more than those; a head dimension that is not native
+    (10, 16, 16, 300, 64),   # more groups than SMs, two of three tiles in descending order
+    (1, 4, 2, 520, 72),      # three of five; a head dimension that is not native
 ])
 def test_causal_order_of_the_reductions(gqa_lib, shape):
-    """The causal list starts with the first four KV tiles of a group in descending order, and the turns follow it.  Three
+    """The causal list starts with half of the KV tiles of a group, four at most, in descending order, and the turns follow it.  Three
     runs bit-identical, dK and dV the default mode's bits, dQ its sums in another order (as above)."""
     B, Hq, Hkv, S, D = shape
     gen = torch.Generator(device="cuda").manual_seed(6)
