@@ -208,7 +208,7 @@ __device__ __forceinline__ uint32_t p_col_of_kstep(int kk) {
 // sequence are skipped by the producer, the rows beyond a sequence's end are masked in P^T.
 // kWithDQ = false: the variant that leaves dQ to the separate query-parallel pass (gqa_bwd_dq_sm100.cu): no dQ
 // product, idle drain warps, and at D = 64 no dS^T in shared memory at all (dK reads its copy in TMEM).
-// kPadded: a head dimension that is not native.
+// kPadded: K steps and columns of nothing but padding are left out (see padded_form).
 template <int D, bool kWithDQ, bool kVarlen, bool kPadded>
 __global__ void __launch_bounds__(BwdCfg<D>::kThreads, 1)
 gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
@@ -417,9 +417,11 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV), q_addr = smem_u32(sQ);
     const uint32_t do_addr = smem_u32(sDO), ds_addr = smem_u32(sDS);
     // Columns of the products.  kPadded: the K steps of S^T and dP^T and the columns of dV, dK and dQ that hold nothing but
-    // padding are left out (the accumulator columns beyond n_cols are never written, and nothing reads them).  Forward and
-    // backward of B2 Hq16 Hkv4 S1024 D80 causal: 122.8 -> 108.9 us on a B200.
-    const int n_cols = kPadded ? (p.d_real + 15) & ~15 : D;
+    // padding are left out.  No product writes the accumulators' columns from n_cols on; what is in them, which need not be a
+    // number, reaches padding columns of dq_accum with the 32-column boxes that begin below n_cols (the finalise kernel reads
+    // the real columns only) and no other memory.  Forward and backward of B2 Hq16 Hkv4 S1024 D80 causal: 122.8 -> 105.8 us on
+    // a B200.
+    const int n_cols = kPadded ? product_cols(p.d_real) : D;
 
     if (warp == Cfg::kWarpTma) {
         // ======================= TMA producer =======================
@@ -798,7 +800,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                 reduce_box(1);
                 stage_box(vc);
                 reduce_box(2);
-                if (n_cols > 96) {  // not all padding
+                if constexpr (!kPadded) {  // (96 columns at most, see padded_form)
                     stage_box(va);
                     reduce_box(3);
                 }
@@ -1014,9 +1016,10 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                     tmem_ld16(tA + ch * 16, v);
                     tmem_wait_ld();
                     if (p.parts > 1) {
+                        const bool any = row_ok && (!kPadded || w * kQuarter + ch * 16 < n_cols);  // of the real columns
 #pragma unroll
                         for (int i = 0; i < 4; ++i)
-                            if (row_ok)
+                            if (any)
                                 *reinterpret_cast<float4*>(pdst + ch * 16 + i * 4) =
                                     make_float4(__uint_as_float(v[4 * i + 0]) * mul, __uint_as_float(v[4 * i + 1]) * mul,
                                                 __uint_as_float(v[4 * i + 2]) * mul, __uint_as_float(v[4 * i + 3]) * mul);
@@ -1164,7 +1167,7 @@ int launch_bwd_t(const void* Q, const void* K, const void* V, const void* dO, co
     if (varlen && (!dq_accum || dq_turn || parts != 1 || !s.bshd || s.B != 1)) return GQA_ERR_BAD_ARGUMENT;
     auto kernel = varlen      ? gqa_bwd_sm100_kernel<D, true, true, false>
                   : !dq_accum ? gqa_bwd_sm100_kernel<D, false, false, false>
-                  : s.D != D  ? gqa_bwd_sm100_kernel<D, true, false, true>
+                  : padded_form(s) ? gqa_bwd_sm100_kernel<D, true, false, true>
                               : gqa_bwd_sm100_kernel<D, true, false, false>;
     const int smem = Cfg::kSmemTotal + (varlen ? (int)sizeof(PackedList) : 0);
     GQA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));

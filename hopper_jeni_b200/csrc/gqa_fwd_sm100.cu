@@ -89,8 +89,8 @@ struct FwdParams {
 
 // What a launch of the kernel has beside the plain case.
 enum Form {
-    kNative,  // head dimension of the kernel, one length for the whole batch
-    kPadded,  // another head dimension: K steps and columns of nothing but padding are left out
+    kNative,  // one length for the whole batch, all columns of the kernel (the ones beyond the head dimension are zeros)
+    kPadded,  // K steps and columns of nothing but padding are left out (see padded_form)
     kPacked,  // packed variable-length batch
 };
 
@@ -375,7 +375,7 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
         const int t = warp - kWarpMma0;
         const uint32_t leader = elect_one() ? 1u : 0u;
         const uint32_t idesc_qk = make_idesc_bf16(128, kHalf, false, false);
-        const int n_cols = kForm == kPadded ? (p.d_real + 15) & ~15 : D;  // columns of Q, K, V that are not all padding
+        const int n_cols = kForm == kPadded ? product_cols(p.d_real) : D;  // columns of Q, K, V that are not all padding
         const uint32_t idesc_pv = make_idesc_bf16(128, n_cols, false, true);
         const uint32_t q_addr = smem_u32(sQ) + t * Cfg::kTileBytes, k_addr = smem_u32(sK), v_addr = smem_u32(sV);
         const uint32_t colS = tmem + (t ? Cfg::kColS1 : Cfg::kColS0), colO = tmem + (t ? Cfg::kColO1 : Cfg::kColO0);
@@ -691,7 +691,7 @@ int launch_fwd_t(const void* Q, const void* K, const void* V, void* O, float* LS
         return more ? gqa_fwd_sm100_kernel<D, F, true> : gqa_fwd_sm100_kernel<D, F, false>;
     };
     auto kernel = s.cu_seqlens ? pick(std::integral_constant<Form, kPacked>{})
-                  : s.D != D   ? pick(std::integral_constant<Form, kPadded>{})
+                  : padded_form(s) ? pick(std::integral_constant<Form, kPadded>{})
                                : pick(std::integral_constant<Form, kNative>{});
     const int smem = Cfg::kSmemTotal + (s.cu_seqlens ? (int)sizeof(PackedList) : 0);
     GQA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));

@@ -65,6 +65,14 @@ int launch_bwd_preprocess(const void* O, const void* dO, const float* lse, float
 int launch_dq_finalise(const float* dq_accum, void* dQ, size_t rows, float scale, cudaStream_t stream,
                        int D, int S_bshd = 0, int H_bshd = 0);
 
+// Columns of a head dimension's products: a K step is 16 wide.
+inline __host__ __device__ int product_cols(int D) { return (D + 15) & ~15; }
+// Whether a head dimension runs in the kernels' padded form, which leaves out the K steps and columns of nothing but padding: its
+// loops have run-time bounds, so it pays from 32 columns on.  B200, forward / backward, time of the plain form over the padded
+// form's, B8 Hq16 Hkv4 S4096 and smaller: 48 or 32 columns left out (D = 32 and 72 to 96) 0.99 to 1.08 / 1.02 to 1.19; 16 (D = 40,
+// 48, 104, 112) 0.97 to 1.01 / 0.97 to 1.02; none (D = 56, 120) 0.96 to 0.99 / 0.96 to 1.01.
+inline bool padded_form(const Shape& s) { return s.Dp() - product_cols(s.D) >= 32; }
+
 // Tensor-core forward (tcgen05 + TMEM + TMA).
 int launch_fwd_sm100(const void* Q, const void* K, const void* V, void* O, float* LSE, const Shape& s,
                      unsigned int* status, cudaStream_t stream);

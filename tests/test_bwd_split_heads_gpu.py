@@ -51,6 +51,24 @@ def test_split_heads_matches_oracle_and_unsplit(gqa_lib, oracle, case):
     assert util.metrics(util.to_np(runs[0][2]), util.to_np(dv1))["rel_rms"] < 2e-3
 
 
+@pytest.mark.parametrize("D", [24, 32, 40, 72, 96, 104])
+def test_split_leaves_padding_columns_alone(gqa_lib, oracle, D):
+    """Head dimensions with and without products over padding, cut by query head, in a workspace full of NaN: only real columns
+    of the partial sums and of the dQ accumulator count."""
+    B, Hq, Hkv, S, causal = 1, 8, 1, 1000, True
+    assert ops.bwd_workspace_bytes(B, Hq, Hkv, S, D, causal, split_heads=True) > ops.bwd_workspace_bytes(B, Hq, Hkv, S, D, causal)
+    q, k, v, do = util.make_inputs(B, Hq, Hkv, S, D, seed=18)
+    sc = util.default_scale(D)
+    tq, tk, tv, tdo = (util.to_dev_bf16(x) for x in (q, k, v, do))
+    o_ref, lse_ref = oracle.forward(q, k, v, causal, sc)
+    to, tlse = util.to_dev_bf16(util.bf16_round(o_ref)), torch.from_numpy(lse_ref).cuda()
+    ws = torch.full((ops.bwd_workspace_bytes(B, Hq, Hkv, S, D, causal, split_heads=True),), 0xFF, dtype=torch.uint8, device="cuda")
+    got = ops.gqa_backward(tq, tk, tv, to, tdo, tlse, causal=causal, scale=sc, workspace=ws, split_heads=True)
+    ops.check_status(ws)
+    for g, want, name in zip(got, oracle.backward(q, k, v, do, causal, sc), ("dQ", "dK", "dV")):
+        util.assert_close_bf16(util.to_np(g), want, name, util.REL_RMS_BWD)
+
+
 def test_split_needs_the_matching_workspace(gqa_lib):
     B, Hq, Hkv, S, D = 1, 8, 1, 1024, 64
     small = ops.bwd_workspace_bytes(B, Hq, Hkv, S, D, True)
