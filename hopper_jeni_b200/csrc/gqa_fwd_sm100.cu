@@ -634,6 +634,20 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     }
 }
 
+// Causal, longest items first: whether single query tiles finish sooner than pairs in a launch of more tiles than SMs.  In units of a
+// quarter of the time that a pair takes for a key block (800 cycles), a single tile takes 3 for it, and a launch of more items
+// than SMs 4 more (see kMore).  As pairs the launch takes as long as its longest one; as single tiles as long as the longest
+// of them, or the SMs' share of all key blocks and a sixth for what list scheduling leaves over.  (With so few items pairs are
+// never bound by their share.)  B200, us, pairs / single tiles: B2 Hq12 S1000 D128 19.9 / 15.9, B1 Hq16 S2048 D128 33.6 / 27.7, D64
+// 30.2 / 24.8, B1 Hq4 S8192 D128 108 / 87, B1 Hq5 S8192 D128 114 / 104, B4 Hq8 S700 D128 16.2 / 13.6, B2 Hq16 S1024 D128 20.4 / 18.8;
+// on the other side of the line B1 Hq36 S1024 D128 20.0 / 20.3, B1 Hq40 S1024 D128 20.8 / 23.7, B1 Hq10 S4096 D64 53.5 / 54.6,
+// B2 Hq32 S512 D128 13.1 / 14.5, B1 Hq6 S8192 D128 115 / 129.
+bool single_tiles(int n_tiles, long long heads, int sms) {
+    const long long n = n_tiles, blocks = heads * n * (n + 1) / 2;
+    const long long longest_pair = n % 2 == 0 ? 4 * n : std::max(4 * (n - 1), 3 * n);
+    return std::max(6 * n * sms, 7 * blocks) + 8LL * sms < 2 * longest_pair * sms;
+}
+
 template <int D>
 int launch_fwd_t(const void* Q, const void* K, const void* V, void* O, float* LSE, const Shape& s, unsigned int* status,
                  cudaStream_t stream) {
@@ -660,9 +674,10 @@ int launch_fwd_t(const void* Q, const void* K, const void* V, void* O, float* LS
     p.bshd = s.bshd;
     p.d_real = s.D;
     p.cu = s.cu_seqlens;
-    // Two query tiles per item share the K/V blocks and keep the tensor core busy in turns; one tile per item finishes
-    // sooner when every tile gets an SM of its own.  B200, D = 128 causal: 128 tiles (B1 Hq16 S1024) 22.5 us as single
-    // tiles against 25.6 us as pairs; 192 tiles (B2 Hq12 S1000) 30.8 against 26.6: the second round costs more.
+    // Two query tiles per item share the K/V blocks and keep the tensor core busy in turns: 3 130 cycles per key block for both,
+    // against 2 450 for one tile alone.  One tile per item finishes sooner when every tile gets an SM of its own (B200, D = 128
+    // causal: 128 tiles, B1 Hq16 S1024, 22.5 us as single tiles against 25.6 us as pairs) and when the longest item bounds the
+    // launch (single_tiles()).
     const int n_tiles = ((s.cu_seqlens ? s.max_seqlen : s.S) + kTile - 1) / kTile, n_seqs = s.cu_seqlens ? s.n_seqs : s.B;
     // Items of a packed batch are listed where that pays and the lengths differ (equal ones are in order as they are: with the
     // list 8 sequences of 300 tokens, Hq16 D128, take 18.4 us instead of 17.3).  Every sequence ends with one partial item at
@@ -674,14 +689,14 @@ int launch_fwd_t(const void* Q, const void* K, const void* V, void* O, float* LS
         const long long all = (long long)((n_tiles + tiles - 1) / tiles) * n_seqs;
         return s.Hq * (p.n_listed ? std::min(all, (long long)s.S / (tiles * kTile) + n_seqs) : all);
     };
-    p.tiles = items(1) <= sm_count() ? 1 : 2;
-    p.n_groups = (n_tiles + p.tiles - 1) / p.tiles;
-    p.scale_log2 = s.scale * kLog2e;
     // Causal items are of very different length: the longest of all heads first keeps the end of the launch short, as long as
     // L2 holds K and V of what runs at a time (head by head they are read from memory once, however long the launch).  B200, us:
     // B1 Hq16 S4096 D128 94.0 -> 65.0, D64 82.2 -> 55.3; B1 Hq32 S2048 D128 71.9 -> 51.5; B16 Hq16 Hkv2 S4096 D64 (34 MB of K and
     // V) 764 -> 737, but B8 Hq32 Hkv8 S8192 D128 (268 MB) 3 968 -> 4 130.
     p.tile_slow = s.causal && !s.cu_seqlens && s.kv_rows() * s.D * 4 <= kOrderKvBytes;
+    p.tiles = items(1) <= sm_count() || (p.tile_slow && single_tiles(n_tiles, (long long)n_seqs * s.Hq, sm_count())) ? 1 : 2;
+    p.n_groups = (n_tiles + p.tiles - 1) / p.tiles;
+    p.scale_log2 = s.scale * kLog2e;
     const dim3 grid = p.n_listed    ? dim3((unsigned)items(p.tiles))
                       : p.tile_slow ? dim3(s.Hq, n_seqs, p.n_groups)
                                     : dim3(p.n_groups, s.Hq, n_seqs);

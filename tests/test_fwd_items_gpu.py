@@ -82,6 +82,27 @@ def test_bits_do_not_depend_on_the_launch(gqa_lib, Hq, Hkv, S, D, causal):
     ops.check_status()
 
 
+@pytest.mark.parametrize("Hq,Hkv,S,D", [
+    (24, 8, 1000, 128),   # 192 single tiles: the longest item bounds the launch
+    (28, 4, 1024, 64),    # 224
+    (36, 6, 1024, 64),    # 288 tiles in pairs: one head more than the line allows
+    (24, 8, 900, 80),     # the last tile holds four rows
+    (64, 8, 600, 128),    # an odd number of tiles, the last one partial
+    (5, 1, 5000, 128),    # 200 single tiles, 40 key blocks in the longest
+])
+def test_single_tiles_and_pairs_are_the_same_bits(gqa_lib, Hq, Hkv, S, D):
+    """Causal launches of more tiles than SMs on both sides of the line between one and two query tiles per item."""
+    gen = torch.Generator(device="cuda").manual_seed(12)
+    q, k, v = (torch.randn(1, h, S, D, generator=gen, device="cuda").bfloat16() for h in (Hq, Hkv, Hkv))
+    o, lse = ops.gqa_forward(q, k, v, causal=True)
+    G = Hq // Hkv
+    for h in range(Hkv):  # a head's shard: every tile gets an SM of its own
+        r = slice(h * G, (h + 1) * G)
+        o_h, lse_h = ops.gqa_forward(q[:, r].contiguous(), k[:, h:h + 1].contiguous(), v[:, h:h + 1].contiguous(), causal=True)
+        assert torch.equal(o_h, o[:, r]) and torch.equal(lse_h, lse[:, r]), h
+    ops.check_status()
+
+
 @pytest.mark.parametrize("causal", [False, True])
 @pytest.mark.parametrize("D", [64, 128])
 def test_items_packed(gqa_lib, D, causal):
