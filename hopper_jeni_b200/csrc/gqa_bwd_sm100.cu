@@ -209,7 +209,9 @@ __device__ __forceinline__ uint32_t p_col_of_kstep(int kk) {
 // kWithDQ = false: the variant that leaves dQ to the separate query-parallel pass (gqa_bwd_dq_sm100.cu): no dQ
 // product, idle drain warps, and at D = 64 no dS^T in shared memory at all (dK reads its copy in TMEM).
 // kPadded: K steps and columns of nothing but padding are left out (see padded_form).
-template <int D, bool kWithDQ, bool kVarlen, bool kPadded>
+// kOrdered: the ordered (deterministic) mode, p.dq_turn given: one warp issues S^T, dP^T and dV, and the one that issues dV
+// otherwise hands the turns on.
+template <int D, bool kWithDQ, bool kVarlen, bool kPadded, bool kOrdered>
 __global__ void __launch_bounds__(BwdCfg<D>::kThreads, 1)
 gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                      const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapDO,
@@ -259,7 +261,8 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(item_full + kItemSlots);
     volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(tmem_slot + 1);
     volatile int* item_slot = reinterpret_cast<volatile int*>(tmem_slot + 2);  // [kItemSlots]
-    static_assert((8 + 3 * Cfg::kQStages + 3 * Cfg::kDOStages + kItemSlots) * 8 + 8 + kItemSlots * 4 <= 384, "barrier area");
+    uint32_t* dq_reduced = tmem_slot + 2 + kItemSlots;  // [4] ordered mode: dQ tiles whose reductions have completed, per drain warp
+    static_assert((8 + 3 * Cfg::kQStages + 3 * Cfg::kDOStages + kItemSlots) * 8 + 8 + kItemSlots * 4 + 16 <= 384, "barrier area");
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
@@ -364,6 +367,11 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     auto q_x_of = [&](const WorkItem& w, int it) { return p.bshd ? head_of(w, it) * D : 0; };
     auto q_z_of = [&](const WorkItem& w, int it) { return p.bshd ? w.b : w.b * p.Hq + head_of(w, it); };
     auto ws_z_of = [&](const WorkItem& w, int it) { return w.b * p.Hq + head_of(w, it); };
+    // Ordered mode: the place of a KV tile in the order of a query tile (which sees the KV tiles up to its own).
+    auto place_of = [&](int kt, int row) -> unsigned int {
+        const int qt = (int)((unsigned)row / kTile);
+        return (unsigned)(kt < p.lead ? min(p.lead - 1, qt) - kt : kt);
+    };
 
     if (tid == 0) {
         mbar_init(kv_full, 1);
@@ -386,6 +394,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
             mbar_init(&do_full[i], 1);
         }
         fence_mbar_init();
+        for (int i = 0; i < 4; ++i) dq_reduced[i] = 0u;
     }
     if (warp == Cfg::kWarpMmaS) {
         tmem_alloc(tmem_slot, Cfg::kTmemCols);
@@ -422,6 +431,16 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     // the real columns only) and no other memory.  Forward and backward of B2 Hq16 Hkv4 S1024 D80 causal: 122.8 -> 105.8 us on
     // a B200.
     const int n_cols = kPadded ? product_cols(p.d_real) : D;
+
+    auto issue_dv = [&](uint32_t leader, int dos, bool accumulate) {
+        const uint32_t idesc = make_idesc_bf16(128, n_cols, false, true);
+        const uint32_t b0 = do_addr + dos * Cfg::kTileBytes;
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)
+            umma_ts_pred(leader, tmem + Cfg::kColDV, tmem + p_col_of_kstep<D>(kk),
+                         make_sdesc_sw128(b0 + kk * 2048, kPanel, 1024), idesc, (accumulate || kk > 0));
+        umma_commit_pred(leader, &p_free[dos]);
+    };
 
     if (warp == Cfg::kWarpTma) {
         // ======================= TMA producer =======================
@@ -545,7 +564,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
             }
         }
     } else if (warp == Cfg::kWarpMmaS) {
-        // ======================= issuer: S^T(it) = K Q^T, dP^T(it) = V dO^T =======================
+        // ======================= issuer: S^T(it) = K Q^T, dP^T(it) = V dO^T; ordered mode: and dV =======================
         // The whole warp runs the loop (uniform control flow); `leader` marks the one lane that issues.
         const uint32_t leader = elect_one() ? 1u : 0u;
         const uint32_t idesc = make_idesc_bf16(128, 128, false, false);
@@ -571,6 +590,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
             if (idx < 0) break;
             const int n_iter = decode(idx).n_iter;
             ok = mbar_wait(kv_full, j & 1, ctx, 20);
+            if (kOrdered && j > 0) ok = ok && mbar_wait(acc_empty, (j - 1) & 1, ctx, 37);
             for (int it = 0; it < n_iter && ok; ++it, ++gi) {
                 const int qs = gi % Cfg::kQStages, dos = gi % Cfg::kDOStages;
                 ok = mbar_wait(&q_full[qs], (gi / Cfg::kQStages) & 1, ctx, 21);
@@ -594,12 +614,18 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                 issue(Cfg::kColDP, v_addr, do_addr + dos * Cfg::kTileBytes, smem_u32(sDltCol) + dos * Cfg::kColPanel);
                 umma_commit_pred(leader, &dp_full[dos]);
                 GQA_TRACE(1, gi, 3);
+                if constexpr (kOrdered) {
+                    ok = mbar_wait(p_ready, gi & 1, ctx, 31);
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    issue_dv(leader, dos, it > 0);
+                    if (it + 1 == n_iter) umma_commit_pred(leader, acc_full);
+                }
             }
         }
-    } else if (warp == Cfg::kWarpMmaDV) {
+    } else if (warp == Cfg::kWarpMmaDV && !kOrdered) {
         // ======================= issuer: dV += P^T dO(it)  (A from TMEM, B = dO read MN-major) =======================
         const uint32_t leader = elect_one() ? 1u : 0u;
-        const uint32_t idesc = make_idesc_bf16(128, n_cols, false, true);
         int gi = 0;
         bool ok = true;
         for (int j = 0; ok; ++j) {
@@ -613,15 +639,45 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                 if (!ok) break;
                 tc_fence_after_sync();
                 GQA_TRACE(3, gi, 0);
-                const uint32_t b0 = do_addr + dos * Cfg::kTileBytes;
-#pragma unroll
-                for (int kk = 0; kk < 8; ++kk)
-                    umma_ts_pred(leader, tmem + Cfg::kColDV, tmem + p_col_of_kstep<D>(kk),
-                                 make_sdesc_sw128(b0 + kk * 2048, kPanel, 1024), idesc, (it > 0 || kk > 0));
-                umma_commit_pred(leader, &p_free[dos]);
+                issue_dv(leader, dos, it > 0);
                 GQA_TRACE(3, gi, 1);
             }
             if (ok) umma_commit_pred(leader, acc_full);
+        }
+    } else if (warp == Cfg::kWarpMmaDV) {
+        // ======================= ordered mode: hands the turns on =======================
+        // A release at GPU scope takes about 1 000 cycles, which the drain warps, the longest role of this mode, do not have.  B200,
+        // us, released by the drain warps / here: B2 Hq24 Hkv8 S4096 D128 causal 803 / 733, without a mask 1 428 / 1 315, B8 Hq12 Hkv4
+        // S4096 D64 causal 953 / 869, B1 Hq64 Hkv8 S8192 D128 causal 4 004 / 3 525, B16 Hq32 Hkv8 S1024 D128 771 / 744.  Lane
+        // l < 4 stands for drain warp l; the four slices of a tile are handed on together.
+        if constexpr (kOrdered) {
+            uint32_t gi = 0;
+            bool ok = true;
+            for (int j = 0; ok; ++j) {
+                const int idx = fetch_item(j);
+                if (idx < 0) break;
+                const WorkItem w = decode(idx);
+                for (int it = 0; it < w.n_iter && ok; ++it, ++gi) {
+                    bool good = true;
+                    if (lane < 4) {
+                        const int row = q_y_of(w, it);
+                        const long long t0 = clock64();
+                        for (uint32_t polls = 0; ld_acquire_cta(&dq_reduced[lane]) <= gi;) {
+                            __nanosleep(64);
+                            if ((++polls & 0x3fu) == 0 && (*abort_flag != 0 || clock64() - t0 > kWaitLimitCycles)) {
+                                good = false;
+                                break;
+                            }
+                        }
+                        if (good) st_release_gpu(p.dq_turn + ((size_t)ws_z_of(w, it) * p.n_tiles + row / kTile) * 4 + lane, place_of(w.kt, row) + 1u);
+                    }
+                    ok = __all_sync(0xffffffffu, good);
+                    if (!ok && lane == 0 && *abort_flag == 0) {
+                        *abort_flag = 44;
+                        atomicCAS(p.status, 0u, 0x80000000u | (44u << 20) | (blockIdx.x & 0xfffffu));
+                    }
+                }
+            }
         }
     } else if (warp == Cfg::kWarpMmaDK) {
         // ======================= issuer: dK += dS^T Q(it)  (A = dS^T K-major, B = Q read MN-major), then dQ(it) =======================
@@ -695,7 +751,8 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
         constexpr bool kDet = decltype(det)::value;
         // Deterministic mode: the reductions into one 32-row slice of the accumulator are applied in the order of the item
         // list.  The CTA whose KV tile is the n-th of them waits until the slice's counter reads n (its predecessors run or
-        // have run: they have smaller block indices), and hands on with n + 1 once its own reductions have completed.
+        // have run: they have smaller block indices), and hands on with n + 1 once its own reductions have completed (the
+        // warp that issues dV in the default mode does).
         auto turn_acquire = [&](unsigned int* turn, unsigned int early, unsigned int mine) -> bool {
             uint32_t good = 1;
             if (lane == 0) {
@@ -716,26 +773,19 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
             }
             return __shfl_sync(0xffffffffu, good, 0) != 0;
         };
-        // The turn of a tile is handed on one iteration later, just before the next tile's reductions are issued:
-        // by then the reductions have had a TMEM round trip and a staging pass to land, so the wait for their
-        // completion is short.  (Holding the turns of three tiles instead was slower: the hand-over delay, not the
-        // wait, is what the CTAs of a group queue on.)
-        // The place of a KV tile in the order of a query tile (which sees the KV tiles up to its own).  Worked out where it is
-        // needed: held in a register, it cost the default path two spilled words.
-        auto place_of = [&](int kt, int row) -> unsigned int {
-            const int qt = (int)((unsigned)row / kTile);
-            return (unsigned)(kt < p.lead ? min(p.lead - 1, qt) - kt : kt);
-        };
-        unsigned int* held = nullptr;  // slice whose turn this warp still holds
-        unsigned int held_next = 0;    // the value that hands it on
-        auto release_held = [&]() {
-            if (kDet && held) {
+        // A tile counts as reduced one iteration later, just before the next tile's reductions are issued: by then its own have
+        // had a TMEM round trip and a staging pass to land, so the wait for their completion is short.  (Counting three tiles
+        // later instead was slower: the hand-over delay, not the wait, is what the CTAs of a group queue on.)
+        [[maybe_unused]] bool pending = false;
+        [[maybe_unused]] uint32_t n_reduced = 0;
+        auto count_reduced = [&]() {
+            if (kDet && pending) {
                 if (lane == 0) {
                     bulk_wait_all();  // completed: the sums are visible to this thread
-                    st_release_gpu(held, held_next);
+                    st_release_cta(&dq_reduced[warp], ++n_reduced);
                 }
                 __syncwarp();
-                held = nullptr;
+                pending = false;
             }
         };
         int gi = 0;
@@ -793,7 +843,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                 tmem_wait_ld();
                 tc_fence_before_sync();
                 mbar_arrive(dq_empty);     // the dP^T columns are free after two TMEM round trips
-                release_held();
+                count_reduced();
                 if (kDet && !turn_mine) turn_mine = turn_acquire(turn, early, place_of(kt, row));
                 reduce_box(0);
                 stage_box(vb);
@@ -804,7 +854,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                     stage_box(va);
                     reduce_box(3);
                 }
-                if (kDet && turn_mine) { held = turn; held_next = place_of(kt, row) + 1u; }
+                if (kDet && turn_mine) pending = true;
             } else {
     #pragma unroll 1
                 for (int rnd = 0; rnd < kRounds; ++rnd) {
@@ -829,7 +879,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                     }
                     fence_proxy_async_smem();
                     __syncwarp();
-                    release_held();
+                    count_reduced();
                     GQA_TRACE(2, gi, 2);
                     if (kDet && !turn_mine) turn_mine = turn_acquire(turn, early, place_of(kt, row));
                     GQA_TRACE(2, gi, 3);
@@ -842,7 +892,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                     }
                     __syncwarp();
                 }
-                if (kDet && turn_mine) { held = turn; held_next = place_of(kt, row) + 1u; }
+                if (kDet && turn_mine) pending = true;
             }
             if (!turn_mine) { going = false; break; }  // a bounded wait gave up: the abort flag is set
             GQA_TRACE(2, gi, 1);
@@ -855,8 +905,10 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
         }
         }
         if (warp == 0) GQA_MARK(7);
-        release_held();
+        count_reduced();
         };
+        // (The default form keeps the ordered loop, which it never takes: with the unordered one alone ptxas schedules the role so
+        // that B2 Hq32 S1537 D128 takes 170 us instead of 166 and B4 Hq32 S1024 D128 143 instead of 140.)
         if (p.dq_turn)
             drain_items(std::true_type{});
         else
@@ -1165,10 +1217,11 @@ int launch_bwd_t(const void* Q, const void* K, const void* V, const void* dO, co
     }
     const bool varlen = s.cu_seqlens != nullptr;
     if (varlen && (!dq_accum || dq_turn || parts != 1 || !s.bshd || s.B != 1)) return GQA_ERR_BAD_ARGUMENT;
-    auto kernel = varlen      ? gqa_bwd_sm100_kernel<D, true, true, false>
-                  : !dq_accum ? gqa_bwd_sm100_kernel<D, false, false, false>
-                  : padded_form(s) ? gqa_bwd_sm100_kernel<D, true, false, true>
-                              : gqa_bwd_sm100_kernel<D, true, false, false>;
+    auto kernel = varlen      ? gqa_bwd_sm100_kernel<D, true, true, false, false>
+                  : !dq_accum ? gqa_bwd_sm100_kernel<D, false, false, false, false>
+                  : dq_turn   ? (padded_form(s) ? gqa_bwd_sm100_kernel<D, true, false, true, true> : gqa_bwd_sm100_kernel<D, true, false, false, true>)
+                  : padded_form(s) ? gqa_bwd_sm100_kernel<D, true, false, true, false>
+                              : gqa_bwd_sm100_kernel<D, true, false, false, false>;
     const int smem = Cfg::kSmemTotal + (varlen ? (int)sizeof(PackedList) : 0);
     GQA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     BwdParams p;

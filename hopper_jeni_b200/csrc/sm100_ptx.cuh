@@ -161,6 +161,16 @@ __device__ __forceinline__ void st_release_gpu(unsigned int* p, unsigned int v) 
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// Flag in shared memory between the warps of a block.
+__device__ __forceinline__ uint32_t ld_acquire_cta(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release_cta(uint32_t* p, uint32_t v) {
+    asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
+}
+
 // ----------------------------------------------------------------------------
 // Programmatic dependent launch.  A kernel launched with launch_after() (gqa_common.cuh) may start while the one before it
 // in the stream still runs, once every block of that one has called pdl_launch_dependents() or ended; pdl_wait() returns when

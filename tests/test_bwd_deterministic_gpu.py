@@ -35,6 +35,25 @@ def test_deterministic_backward_matches_oracle(gqa_lib, oracle, shape, causal):
 
 
 @pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("shape", [
+    (1, 4, 2, 100, 64),     # one tile: a single turn
+    (2, 4, 2, 333, 40),
+    (1, 6, 2, 333, 80),     # the padded form
+    (1, 8, 1, 129, 128),    # the second tile holds one row
+])
+def test_ordered_form_matches_oracle_at_odd_sizes(gqa_lib, oracle, shape, causal):
+    B, Hq, Hkv, S, D = shape
+    (q, k, v, do), (tq, tk, tv, tdo, o, lse) = _inputs(B, Hq, Hkv, S, D, causal, seed=73)
+    refs = oracle.backward(q, k, v, do, causal, util.default_scale(D))
+    ws = torch.full((ops.bwd_workspace_bytes(B, Hq, Hkv, S, D, causal),), 255, dtype=torch.uint8, device="cuda")
+    runs = [ops.gqa_backward(tq, tk, tv, o, tdo, lse, causal=causal, workspace=ws, deterministic=True) for _ in range(2)]
+    ops.check_status(ws)
+    for name, a, b, ref in zip(("dQ", "dK", "dV"), *runs, refs):
+        assert torch.equal(a, b), name
+        util.assert_close_bf16(util.to_np(a), ref, name, util.REL_RMS_BWD)
+
+
+@pytest.mark.parametrize("causal", [False, True])
 @pytest.mark.parametrize("shape", [(2, 12, 4, 2048, 64), (2, 8, 2, 2048, 128), (8, 12, 4, 4096, 64)])
 def test_deterministic_backward_is_bit_reproducible(gqa_lib, shape, causal):
     """More thread blocks than SMs, several per (batch, KV head) group: every dQ tile gets up to S/128 ordered
