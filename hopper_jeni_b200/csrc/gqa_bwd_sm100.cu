@@ -713,8 +713,10 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                     GQA_TRACE(4, gi, 1);
                 };
                 auto issue_dq = [&]() -> bool {  // A = dS^T read MN-major, B = K read MN-major
-                    if (gi > 0 && !mbar_wait(dq_empty, (gi - 1) & 1, ctx, 36)) return false;
-                    tc_fence_after_sync();
+                    if constexpr (!Cfg::kDqAliasesDp) {  // (else dP^T(it) was issued behind that wait, and dS^T(it) comes from it)
+                        if (gi > 0 && !mbar_wait(dq_empty, (gi - 1) & 1, ctx, 36)) return false;
+                        tc_fence_after_sync();
+                    }
                     GQA_TRACE(4, gi, 2);
                     const uint32_t idesc_dq = make_idesc_bf16(128, n_cols, true, true);
 #pragma unroll
@@ -817,13 +819,19 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
             constexpr int kRounds = D / (32 * Cfg::kDqBoxes);
             if constexpr (Cfg::kDrainEarlyRelease) {
                 static_assert(!Cfg::kDrainEarlyRelease || (D == 128 && Cfg::kDqBoxes == 1), "four 32-column chunks, one box");
-                auto stage_box = [&](const uint32_t (&v)[32]) {
+                auto fill_box = [&](const uint32_t (&v)[32]) {
 #pragma unroll
                     for (int c8 = 0; c8 < 8; ++c8)
                         *reinterpret_cast<uint4*>(stage + ((c8 ^ sw) << 4)) =
                             make_uint4(v[4 * c8], v[4 * c8 + 1], v[4 * c8 + 2], v[4 * c8 + 3]);
+                };
+                auto box_filled = [&]() {
                     fence_proxy_async_smem();
                     __syncwarp();
+                };
+                auto stage_box = [&](const uint32_t (&v)[32]) {
+                    fill_box(v);
+                    box_filled();
                 };
                 auto reduce_box = [&](int chunk) {  // then wait until the box may be overwritten
                     if (turn_mine && lane == 0) {
@@ -838,11 +846,18 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                 tmem_ld32(tDQ + 32, vb);
                 tmem_ld32(tDQ + 64, vc);
                 tmem_wait_ld();
-                stage_box(va);
-                tmem_ld32(tDQ + 96, va);  // chunk 0 is in shared memory: its registers take chunk 3
-                tmem_wait_ld();
-                tc_fence_before_sync();
-                mbar_arrive(dq_empty);     // the dP^T columns are free after two TMEM round trips
+                if constexpr (kPadded) {  // three chunks at the most (see padded_form): the dP^T columns are free
+                    tc_fence_before_sync();
+                    mbar_arrive(dq_empty);
+                    stage_box(va);
+                } else {
+                    fill_box(va);
+                    tmem_ld32(tDQ + 96, va);  // chunk 0 is in shared memory: its registers take chunk 3
+                    tmem_wait_ld();
+                    tc_fence_before_sync();
+                    mbar_arrive(dq_empty);     // the dP^T columns are free after two TMEM round trips
+                    box_filled();
+                }
                 count_reduced();
                 if (kDet && !turn_mine) turn_mine = turn_acquire(turn, early, place_of(kt, row));
                 reduce_box(0);
@@ -1121,11 +1136,14 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                 ok = make_p(gi, p.causal && qi == 0, qi == n_qt - 1 ? q_tail : kTile, kv_valid);
                 if (++qi == n_qt) qi = 0;
                 if (!ok) break;
-                ok = mbar_wait(&dp_full[gi % Cfg::kDOStages], (gi / Cfg::kDOStages) & 1, ctx, 53);
-                if (ok && gi > 0) {  // dK and dQ of the iteration before have read its dS^T: the later of the two has completed
+                // (A wait costs 100 to 150 cycles also when it is over, so the one that takes time comes last.  With it first, another
+                // wait in front of dQ at D = 128 and the box of dQ's first chunk handed over before its columns were, B1 Hq8 Hkv2
+                // S2048 D128 took 171 us instead of 169, B2 Hq32 S1537 D128 167.0 instead of 165.2.)
+                if (gi > 0) {  // dK and dQ of the iteration before have read its dS^T: the later of the two has completed
                     if constexpr (kWithDQ && !Cfg::kDqFirst) ok = mbar_wait(dq_full, (gi - 1) & 1, ctx, 54);
                     else ok = mbar_wait(&dk_done[(gi - 1) % Cfg::kQStages], ((gi - 1) / Cfg::kQStages) & 1, ctx, 54);
                 }
+                ok = ok && mbar_wait(&dp_full[gi % Cfg::kDOStages], (gi / Cfg::kDOStages) & 1, ctx, 53);
                 if (!ok) break;
                 tc_fence_after_sync();
                 if (trace_me) GQA_TRACE(0, gi, 0);
