@@ -173,6 +173,8 @@ struct BwdCfg {
 };
 
 struct BwdParams {
+    const uint4* lse_cols;  // the -LSE/scale and -Delta columns, 16 bytes per query row (see mapLseCol, mapDltCol)
+    const uint4* delta_cols;
     float* dq_accum;     // [B*Hq*S, D] fp32, zeroed by the preprocess stage
     __nv_bfloat16* dK;
     __nv_bfloat16* dV;
@@ -495,6 +497,15 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                     }
                 }
             };
+            // 128 rows of 16 bytes are 2 KB in one piece, which the copy engine takes in 128-byte lines; described as a box it takes
+            // them row by row, and at D = 128 loads and dQ reductions keep it busy all the time (256 of 1 280 rows per tile pair).
+            // Beyond the end of the matrix (queries that must read as zeros) the box is needed.  B200, us, boxes / in one
+            // piece: B1 Hq8 Hkv2 S2048 D128 169.6 / 165.0, B8 Hq12 Hkv4 S4096 D128 2 036 / 2 006, D64 1 215 / 1 202, B2 Hq16 S1024 D80 causal
+            // 84.5 / 82.7.
+            auto load_cols = [&](uint8_t* dst, const uint4* cols, const CUtensorMap* map, uint64_t* bar, int y, int z) {
+                if (y + kTile <= p.S) bulk_load(dst, cols + (size_t)z * p.S + y, Cfg::kColPanel, bar);
+                else tma_load_3d(dst, map, bar, 0, y, z);
+            };
             int idx = blockIdx.x;
             if constexpr (kVarlen) {
                 idx = idx < items() ? place(idx) : -1;
@@ -546,7 +557,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                         mbar_expect_tx(&q_full[st], Cfg::kTileBytes + Cfg::kColPanel);
                         for (int pn = 0; pn < Cfg::kPanels; ++pn)
                             tma_load_3d(sQ + st * Cfg::kTileBytes + pn * kPanel, &mapQ, &q_full[st], qx + pn * 64, qy, qz);
-                        tma_load_3d(sLseCol + st * Cfg::kColPanel, &mapLseCol, &q_full[st], 0, qy, wz);
+                        load_cols(sLseCol + st * Cfg::kColPanel, p.lse_cols, &mapLseCol, &q_full[st], qy, wz);
                     }
                     {
                         const int st = gi % Cfg::kDOStages;
@@ -557,7 +568,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                         mbar_expect_tx(&do_full[st], Cfg::kTileBytes + Cfg::kColPanel);
                         for (int pn = 0; pn < Cfg::kPanels; ++pn)
                             tma_load_3d(sDO + st * Cfg::kTileBytes + pn * kPanel, &mapDO, &do_full[st], qx + pn * 64, qy, qz);
-                        tma_load_3d(sDltCol + st * Cfg::kColPanel, &mapDltCol, &do_full[st], 0, qy, wz);
+                        load_cols(sDltCol + st * Cfg::kColPanel, p.delta_cols, &mapDltCol, &do_full[st], qy, wz);
                     }
                 }
                 idx = next;
@@ -1243,6 +1254,8 @@ int launch_bwd_t(const void* Q, const void* K, const void* V, const void* dO, co
     const int smem = Cfg::kSmemTotal + (varlen ? (int)sizeof(PackedList) : 0);
     GQA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     BwdParams p;
+    p.lse_cols = static_cast<const uint4*>(lse_cols);
+    p.delta_cols = static_cast<const uint4*>(delta_cols);
     p.dq_accum = dq_accum;
     p.dK = static_cast<__nv_bfloat16*>(dK);
     p.dV = static_cast<__nv_bfloat16*>(dV);
