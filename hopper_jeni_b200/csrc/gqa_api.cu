@@ -129,6 +129,11 @@ extern "C" size_t gqa_bwd_workspace_bytes_ex(int B, int Hq, int Hkv, int S, int 
 
 namespace {
 
+bool overlap(const void* a, size_t a_bytes, const void* b, size_t b_bytes) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x < y + b_bytes && y < x + a_bytes;
+}
+
 // Shared body of gqa_bwd and gqa_bwd_stage_times; `ev` is null or four events recorded around the stages.
 int run_bwd(const void* Q, const void* K, const void* V, const void* O, const void* dO, const float* LSE, void* dQ,
             void* dK, void* dV, int B, int Hq, int Hkv, int S, int D, int causal, float scale, void* workspace,
@@ -167,8 +172,10 @@ int run_bwd(const void* Q, const void* K, const void* V, const void* O, const vo
     float* dq_accum = reinterpret_cast<float*>(w + ws.dq_accum_off);
     float* delta_f32 = reinterpret_cast<float*>(w + ws.delta_f32_off);
     // The dQ path.  Default: fp32 TMA reduce-add of the main kernel's dQ tiles into the accumulator: measured faster
-    // than the separate query-parallel pass at every benchmark shape (1.3-1.7x), and so is its ordered (deterministic)
-    // form except at one shape, so the separate pass is taken only when asked for.
+    // than the separate query-parallel pass wherever the KV tiles fill the chip (1.3-1.6x).  Where they leave more than half of
+    // the SMs idle the separate pass, beside the main kernel, takes 0.8 to 0.93 of the default's time in one stream, but 1.3 to
+    // 1.6 of it in four streams that fill the chip together (it does half as many products again), so it is taken only when
+    // asked for.
     const bool dq_separate = (flags & GQA_BWD_DQ_SEPARATE) != 0;
     unsigned int* dq_turn = nullptr;
     if ((flags & GQA_BWD_DETERMINISTIC) && !dq_separate) dq_turn = reinterpret_cast<unsigned int*>(w + ws.dq_turn_off);
@@ -187,8 +194,12 @@ int run_bwd(const void* Q, const void* K, const void* V, const void* O, const vo
         rc = gqa::launch_dkdv_reduce(partial, dK, dV, s, parts, stream);
         if (rc) return rc;
     }
+    // (the main kernel may not run beside a pass that writes what it reads: dQ in place of an input)
+    const size_t q_bytes = s.q_rows() * D * 2, kv_bytes = s.kv_rows() * D * 2;
+    const bool beside = parts == 1 && !overlap(dQ, q_bytes, Q, q_bytes) && !overlap(dQ, q_bytes, dO, q_bytes) &&
+                        !overlap(dQ, q_bytes, K, kv_bytes) && !overlap(dQ, q_bytes, V, kv_bytes);
     if (dq_separate)
-        rc = gqa::launch_bwd_dq_sm100(Q, K, V, dO, LSE, delta_f32, dQ, s, status, stream);
+        rc = gqa::launch_bwd_dq_sm100(Q, K, V, dO, LSE, delta_f32, dQ, s, status, beside, stream);
     else
         rc = gqa::launch_dq_finalise(dq_accum, dQ, s.q_rows(), scale, stream, D, s.bshd ? S : 0, s.bshd ? Hq : 0);
     if (rc) return rc;

@@ -179,6 +179,7 @@ struct BwdParams {
     __nv_bfloat16* dK;
     __nv_bfloat16* dV;
     unsigned int* status;
+    unsigned int* prep_seen;  // see the variant without the dQ part
     unsigned int* dq_turn;  // deterministic mode: one counter per 32 query rows (zeroed), else nullptr
     // Head split: with `parts` > 1 a KV tile's work is cut over `parts` thread blocks, each looping over G / parts
     // of the group's query heads and storing its dK / dV sums as fp32 into `partial` ([part][dV, dK][key row][D of
@@ -409,6 +410,15 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     }
     // Everything above overlaps the end of the preprocess kernel, whose output (workspace) is first used from here on.
     pdl_wait();
+    if constexpr (!kWithDQ) {
+        // The separate dQ pass comes up beside this kernel, on the SMs that it leaves idle, and reads what the preprocess
+        // kernel wrote: `prep_seen` hands that on (this thread has seen it, the pass acquires the word).  Every block is
+        // resident by then, and none waits for the pass.
+        if (tid == 0) {
+            if (blockIdx.x == 0) st_release_gpu(p.prep_seen, 1u);
+            pdl_launch_dependents();
+        }
+    }
     // a thread block of this launch that has already given up leaves a non-zero status word: the blocks that
     // start after it skip their work (see below), so a wedged launch drains in one wave
     if (tid == 0) *abort_flag = (*reinterpret_cast<volatile unsigned int*>(p.status) != 0u) ? 98u : 0u;
@@ -454,7 +464,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
             tma_prefetch_desc(&mapDQ);
             tma_prefetch_desc(&mapLseCol);
             tma_prefetch_desc(&mapDltCol);
-            unsigned int* work_counter = p.status + 16;  // zeroed with the status word before every launch
+            unsigned int* work_counter = p.status + kWorkCounterWord;  // zeroed with the status word before every launch
             int gi = 0;  // iterations issued so far, over all items: the rings and their barriers carry on across items
             // Packed batch: the list runs over super-groups of `run` sequences with all their KV heads, the longest sequences
             // first, in the causal or the non-causal order inside, each laid out for its longest sequence.  (Without the
@@ -521,7 +531,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                     // kernel of another stream then finds no SM to run on.  Four streams of B1 Hq8 Hkv2 S2048 D64 (32
                     // items each), per call of one: 112 us, 229 with the trigger at the start of the block, 117 without
                     // dependent launches; one stream alone 103.5, 103.4 and 109.
-                    pdl_launch_dependents();
+                    if constexpr (kWithDQ) pdl_launch_dependents();
                     break;
                 }
                 const WorkItem w = decode(idx);
@@ -1250,7 +1260,7 @@ int launch_bwd_t(const void* Q, const void* K, const void* V, const void* dO, co
     const bool varlen = s.cu_seqlens != nullptr;
     if (varlen && (!dq_accum || dq_turn || parts != 1 || !s.bshd || s.B != 1)) return GQA_ERR_BAD_ARGUMENT;
     auto kernel = varlen      ? gqa_bwd_sm100_kernel<D, true, true, false, false>
-                  : !dq_accum ? gqa_bwd_sm100_kernel<D, false, false, false, false>
+                  : !dq_accum ? (padded_form(s) ? gqa_bwd_sm100_kernel<D, false, false, true, false> : gqa_bwd_sm100_kernel<D, false, false, false, false>)
                   : dq_turn   ? (padded_form(s) ? gqa_bwd_sm100_kernel<D, true, false, true, true> : gqa_bwd_sm100_kernel<D, true, false, false, true>)
                   : padded_form(s) ? gqa_bwd_sm100_kernel<D, true, false, true, false>
                               : gqa_bwd_sm100_kernel<D, true, false, false, false>;
@@ -1263,6 +1273,7 @@ int launch_bwd_t(const void* Q, const void* K, const void* V, const void* dO, co
     p.dK = static_cast<__nv_bfloat16*>(dK);
     p.dV = static_cast<__nv_bfloat16*>(dV);
     p.status = status;
+    p.prep_seen = status + kPrepSeenWord;
     p.dq_turn = dq_turn;
     p.partial = partial;
     p.parts = parts;

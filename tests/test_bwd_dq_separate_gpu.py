@@ -67,3 +67,31 @@ def test_separate_dq_at_the_headline_shape(gqa_lib):
     assert torch.equal(dk_a, dk_b) and torch.equal(dv_a, dv_b)
     m = util.metrics(util.to_np(dq_b[:2]), util.to_np(dq_a[:2]))
     assert m["rel_rms"] < 3e-3 and m["gate_ok"], m
+
+
+@pytest.mark.parametrize("S", [65, 127, 129, 257, 385, 513])
+@pytest.mark.parametrize("D,causal,layout", [(64, True, "bhsd"), (128, False, "bhsd"), (80, True, "bhsd"), (32, False, "bhsd"),
+                                             (128, True, "bshd")])
+def test_separate_dq_at_tile_edges(gqa_lib, oracle, S, D, causal, layout):
+    """One to five key blocks: the two S buffers, the key ring of three blocks and the value ring of two wrap, the last block and
+    the last tile are partial; padded head dimensions.  dQ written over dO is the same bits (the pass then waits for the main
+    kernel instead of running beside it)."""
+    B, Hq, Hkv = 2, 4, 2
+    q, k, v, do = util.make_inputs(B, Hq, Hkv, S, D, seed=31)
+    sc = util.default_scale(D)
+    o_ref, lse_ref = oracle.forward(q, k, v, causal, sc)
+    order = (lambda t: t.transpose(1, 2).contiguous()) if layout == "bshd" else (lambda t: t)
+    tq, tk, tv, tdo, to = (order(util.to_dev_bf16(x)) for x in (q, k, v, do, util.bf16_round(o_ref)))
+    tlse = torch.from_numpy(lse_ref).cuda()
+    ws = torch.empty(ops.bwd_workspace_bytes(B, Hq, Hkv, S, D, causal), dtype=torch.uint8, device="cuda")
+    kw = dict(causal=causal, scale=sc, workspace=ws, layout=layout)
+    dq, dk, dv = ops.gqa_backward(tq, tk, tv, to, tdo, tlse, dq=torch.full_like(tq, float("nan")), dq_separate=True, **kw)
+    ops.check_status(ws)
+    dq0, dk0, dv0 = ops.gqa_backward(tq, tk, tv, to, tdo, tlse, **kw)
+    assert torch.equal(dk, dk0) and torch.equal(dv, dv0)
+    dq_ref, _, _ = oracle.backward(q, k, v, do, causal, sc)
+    util.assert_close_bf16(util.to_np(order(dq)), dq_ref, "dQ", util.REL_RMS_BWD)
+    over = tdo.clone()
+    dq1, dk1, dv1 = ops.gqa_backward(tq, tk, tv, to, over, tlse, dq=over, dq_separate=True, **kw)
+    ops.check_status(ws)
+    assert torch.equal(dq1, dq) and torch.equal(dk1, dk) and torch.equal(dv1, dv)
