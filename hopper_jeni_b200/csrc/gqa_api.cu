@@ -172,7 +172,7 @@ int run_bwd(const void* Q, const void* K, const void* V, const void* O, const vo
     float* dq_accum = reinterpret_cast<float*>(w + ws.dq_accum_off);
     float* delta_f32 = reinterpret_cast<float*>(w + ws.delta_f32_off);
     // The dQ path.  Default: fp32 TMA reduce-add of the main kernel's dQ tiles into the accumulator: measured faster
-    // than the separate query-parallel pass wherever the KV tiles fill the chip (1.3-1.6x).  Where they leave more than half of
+    // than the separate query-parallel pass wherever the KV tiles fill the chip (1.3-1.7x).  Where they leave more than half of
     // the SMs idle the separate pass, beside the main kernel, takes 0.8 to 0.93 of the default's time in one stream, but 1.3 to
     // 1.6 of it in four streams that fill the chip together (it does half as many products again), so it is taken only when
     // asked for.

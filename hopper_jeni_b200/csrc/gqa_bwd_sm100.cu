@@ -25,7 +25,8 @@
 //   warps 0-3    drain dQ tiles from TMEM into the fp32 accumulator
 //   warps 4-19   four elementwise warpgroups; each owns 32 query columns of the tile pair
 //   warp  20     TMA producer
-//   warps 21-23  UMMA issuers: [S^T, dP^T] | dV | [dK, dQ] (dQ first at D = 128)
+//   warps 21-23  UMMA issuers: [S^T, dP^T] | dV | [dK, dQ] (dQ first at D = 128); ordered mode: [S^T, dP^T, dV] | hands on the
+//                turns of the dQ reductions | [dK, dQ]
 // The five GEMMs wait on different producers, and one issuing warp sustains a 128x64x16 product
 // only every 57 cycles (78 when A comes from TMEM) against 32 cycles of tensor math, so they are
 // issued by three warps in parallel, each a warp-uniform loop with one elected lane; mbarriers
@@ -298,6 +299,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     // 4 487 / 4 423 / 4 578, B4 Hq32 Hkv8 S1024 D128 227 / 192 / 224, B16 Hq32 Hkv8 S1024 D128 767 / 790 / 830.  Of a few tiles
     // half (lead 0 / half / all): B14 Hkv8 S283 D64 174.5 / 176.6 / 180.9, B16 Hkv4 S384 D64 56.1 / 50.2 / 58.0.  It costs 2 to 3 % at
     // the most.  (As many as find an SM at once, which makes the bits depend on the launch: 746, 708, 50; 4 348, 192, 768.)
+    // Since the turns are handed on by a warp of their own, lead 4 / 8: the first shape 731 / 712, B8 Hq32 S4096 3 865 / 4 031.
     struct WorkItem {
         int kt, grp, part, b, hkv, qt0, n_qt, n_iter, kv_x, kv_z;
         int shift;  // the item's loop over the query tiles of a head starts at tile qt0 + shift and wraps around

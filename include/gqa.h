@@ -125,7 +125,7 @@ int gqa_bwd(const void* Q, const void* K, const void* V, const void* O, const vo
  * GQA_BWD_DQ_SEPARATE: compute dQ in a separate query-parallel pass (one thread block per 128-row query tile looping
  * over the key tiles, as the reference's first generations do, src/attention/GQA_bwd.cu:29, :415, :1416) instead
  * of accumulating the main kernel's dQ tiles with fp32 reductions.  S and dP are then computed twice, but dQ needs
- * no accumulator, no finalise pass, and is bit-reproducible by construction.  Measured 1.3-1.6x slower than the
+ * no accumulator, no finalise pass, and is bit-reproducible by construction.  Measured 1.3-1.7x slower than the
  * default where the KV tiles (B * Hkv * ceil(S / 128)) fill the chip.  It runs on the SMs that they leave idle: with fewer
  * than 50 of them, or 100 with a causal mask, a call takes 0.80 to 0.95 of the default's time, if no other stream wants
  * those SMs.  No mode selects it by itself.  Same workspace size.
