@@ -82,8 +82,14 @@ gqa_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_c
                         const DqParams p) {
     using Cfg = DqCfg<D>;
     extern __shared__ __align__(1024) uint8_t smem[];
+    // The next kernel of the stream waits for this one: so that it waits for the main kernel too, the last block does, on every
+    // way out (the others leave their SMs to blocks that have not started).
+    auto wait_for_main = [&]() {
+        if (threadIdx.x == 0 && blockIdx.x + 1 == gridDim.x && blockIdx.y + 1 == gridDim.y && blockIdx.z + 1 == gridDim.z) pdl_wait();
+    };
     if ((smem_u32(smem) & 1023u) != 0) {  // swizzled panels need 1024-byte alignment; report instead of computing garbage
         if (threadIdx.x == 0) atomicCAS(p.status, 0u, 0x80000000u | (99u << 20));
+        wait_for_main();
         return;
     }
     uint8_t* sQ = smem + Cfg::kOffQ;
@@ -159,6 +165,7 @@ gqa_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_c
     const uint32_t tmem = *tmem_slot;
     if (*abort_flag != 0) {  // uniform: every thread reads the flag after the barrier
         if (warp == kWarpMma) tmem_dealloc(tmem, Cfg::kTmemCols);
+        wait_for_main();
         return;
     }
 
@@ -315,9 +322,7 @@ gqa_bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_c
     // ---- teardown ---------------------------------------------------------------
     tc_fence_before_sync();
     __syncthreads();
-    // The next kernel of the stream waits for this one: so that it waits for the main kernel too, the last block does (the
-    // others leave their SMs to blocks that have not started).
-    if (tid == 0 && blockIdx.x + 1 == gridDim.x && blockIdx.y + 1 == gridDim.y && blockIdx.z + 1 == gridDim.z) pdl_wait();
+    wait_for_main();
     if (warp == kWarpMma) {
         if (*abort_flag != 0) abort_grace_period();  // in-flight copies and MMAs land before TMEM is released
         tmem_dealloc(tmem, Cfg::kTmemCols);
