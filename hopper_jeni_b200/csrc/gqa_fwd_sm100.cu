@@ -1,7 +1,7 @@
 // GQA forward for sm_100a: O = softmax(scale * Q K^T [+ causal]) V, LSE.
 //
-// A work item is two 128-row query tiles (one, where every tile gets an SM of its own) of one (batch, query
-// head); the KV head's 128-row key/value blocks stream through a TMA ring.  A thread block works through
+// A work item is two 128-row query tiles (one, where every tile gets an SM of its own, and for the longest tiles of some causal
+// launches) of one (batch, query head); the KV head's 128-row key/value blocks stream through a TMA ring.  A thread block works through
 // several items (see the work-item comment).  Roles:
 //   warps 0-3  softmax warpgroup for query tile 0 (thread = query row = TMEM lane)
 //   warps 4-7  softmax warpgroup for query tile 1
@@ -81,6 +81,7 @@ struct FwdParams {
     int Hq, Hkv, S, causal, bshd;
     int tiles, n_groups;  // query tiles per item (1 or 2), items per (sequence, query head)
     int tile_slow;        // the place in the sequence is the slowest index of the items (x = head, y = sequence, z = place)
+    int singles;          // ... and so many of its last tiles are items of their own (see SingleTiles)
     const int* cu;     // packed variable-length batch: sequence starts (z of an item = sequence), else null
     int n_listed;      // packed batch with a work list (x of an item = place in the list): the sequences in it, else 0
     int d_real;        // head dimension of the tensors (<= D of the kernel; the columns beyond it read as zeros)
@@ -97,7 +98,10 @@ enum Form {
 // kMore: the launch has more items than SMs, so blocks ask for further ones; without it the kernel is the plain
 // one-item-per-block form (every running count below is a constant 0 there): a launch of the kMore form that has nothing to
 // hand out is 1.5 us slower at B1 Hq4 S128 D64 (8.2 against 6.7 us) and 3 % at B2 Hq12 S1000 D128.
-template <int D, Form kForm, bool kMore>
+// kAlone: causal, some of a head's tiles are items of their own and the others pairs (see SingleTiles).  A form of its own because the
+// others are 1 to 3 % slower with that in their item arithmetic (B16 Hq16 Hkv2 S2048 D64 364 -> 375 us, B8 Hq12 Hkv4 S4096 D64 causal
+// 286 -> 293).
+template <int D, Form kForm, bool kMore, bool kAlone>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                      const __grid_constant__ CUtensorMap mapV, const FwdParams p) {
@@ -158,14 +162,14 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     // end of the work list has n_tiles = 0 and no key blocks; the producer passes most of them over, and every role does
     // nothing in one.
     [[maybe_unused]] PackedList* list = reinterpret_cast<PackedList*>(smem + Cfg::kOffList);
-    auto item_at = [&](int hq, int q0, int b, int y0, int len) -> Item {
+    auto item_at = [&](int hq, int q0, int b, int y0, int len, bool pair) -> Item {
         Item w;
         w.hq = hq;
         w.q0 = q0;
         w.b = b;
         w.y0 = y0;
         w.len = len;
-        w.n_tiles = w.q0 >= w.len ? 0 : (p.tiles == 2 && w.q0 + kTile < w.len) ? 2 : 1;
+        w.n_tiles = w.q0 >= w.len ? 0 : (pair && w.q0 + kTile < w.len) ? 2 : 1;
         const int n_blocks_all = (w.len + kTile - 1) / kTile;  // the last block may be partial: keys at and beyond len are masked
         w.n_blk0 = (w.n_tiles == 0) ? 0 : p.causal ? (w.q0 / kTile + 1) : n_blocks_all;
         w.n_blk1 = (w.n_tiles == 2) ? (p.causal ? (w.q0 / kTile + 2) : n_blocks_all) : 0;
@@ -184,18 +188,22 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                 y = r / n_groups;
                 x = r % n_groups;
             }
-        } else if (p.tile_slow) {
+        } else if (kAlone || p.tile_slow) {
             const int place = z;
             z = y;
             y = x;
             x = place;
         }
+        if constexpr (kAlone) {  // the last p.singles tiles of a head one by one, the others in pairs
+            const bool pair = x >= p.singles;
+            return item_at(y, (pair ? 2 * (n_groups - 1 - x) : 2 * n_groups - p.singles - 1 - x) * kTile, z, 0, p.S, pair);
+        }
         const int q0 = (p.causal ? (n_groups - 1 - x) : x) * p.tiles * kTile;  // heavy causal tiles first
         if constexpr (kForm == kPacked) {
             const int y0 = p.cu[z];
-            return item_at(y, q0, 0, y0, p.cu[z + 1] - y0);
+            return item_at(y, q0, 0, y0, p.cu[z + 1] - y0, p.tiles == 2);
         } else {
-            return item_at(y, q0, z, 0, p.S);
+            return item_at(y, q0, z, 0, p.S, p.tiles == 2);
         }
     };
     // The j-th item of this block, published by the producer; false = no more (or give up).  In the plain form every role
@@ -215,7 +223,7 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
             mbar_arrive(&item_empty[sl]);
             if (x < 0) return false;
             if constexpr (kForm == kPacked) {
-                w = item_at(x, y, 0, z, len);
+                w = item_at(x, y, 0, z, len, p.tiles == 2);
                 return true;
             }
         }
@@ -634,19 +642,51 @@ gqa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     }
 }
 
-// Causal, longest items first: whether single query tiles finish sooner than pairs in a launch of more tiles than SMs.  In units of a
-// quarter of the time that a pair takes for a key block (800 cycles), a single tile takes 3 for it, and a launch of more items
-// than SMs 4 more (see kMore).  As pairs the launch takes as long as its longest one; as single tiles as long as the longest
-// of them, or the SMs' share of all key blocks and a sixth for what list scheduling leaves over.  (With so few items pairs are
-// never bound by their share.)  B200, us, pairs / single tiles: B2 Hq12 S1000 D128 19.9 / 15.9, B1 Hq16 S2048 D128 33.6 / 27.7, D64
-// 30.2 / 24.8, B1 Hq4 S8192 D128 108 / 87, B1 Hq5 S8192 D128 114 / 104, B4 Hq8 S700 D128 16.2 / 13.6, B2 Hq16 S1024 D128 20.4 / 18.8;
-// on the other side of the line B1 Hq36 S1024 D128 20.0 / 20.3, B1 Hq40 S1024 D128 20.8 / 23.7, B1 Hq10 S4096 D64 53.5 / 54.6,
-// B2 Hq32 S512 D128 13.1 / 14.5, B1 Hq6 S8192 D128 115 / 129.
-bool single_tiles(int n_tiles, long long heads, int sms) {
-    const long long n = n_tiles, blocks = heads * n * (n + 1) / 2;
-    const long long longest_pair = n % 2 == 0 ? 4 * n : std::max(4 * (n - 1), 3 * n);
-    return std::max(6 * n * sms, 7 * blocks) + 8LL * sms < 2 * longest_pair * sms;
-}
+// Causal launches of more query tiles than SMs, longest items first: how many of a head's last tiles are items of their own, the
+// rest being pairs.  A pair takes 3 130 cycles per key block and one tile alone 2 450, so where the longest pair bounds the launch
+// (bound_by_longest) it ends sooner with that pair's tiles on two SMs.  They then take 1.57 times as much of the SMs' time, which an
+// idle chip has and one with several streams has not: so only as many tiles stand alone as shorten the launch.
+// Units of 800 cycles: a key block of a pair takes 4 and a pair 3 more, one of a single tile 3 and the tile 2 more; of more items than
+// SMs the ones of the second round start when the shortest of the first round end.
+// B200, graph replays, us per launch of a stream with one / two / four streams, all pairs; this rule; all single tiles: B2 Hq12 S1000
+// D128 (4 of 8 tiles) 20.7 / 21.7 / 38; 16.4 / 24.8 / 48; 17.1 / 28.1 / 55.  B1 Hq16 S2048 D128 (6 of 16) 35 / 39 / 74; 29 / 48 / 93;
+// 29 / 54 / 107.  B1 Hq4 S8192 D128 (18 of 64) 110 / 114 / 212; 91 / 136 / 263; 91 / 161 / 318.  B4 Hq8 S700 D128 (2 of 6) 16.6 / 17.9 /
+// 32.8; 13.8 / 20.2 / 38.7; 14.3 / 24.3 / 47.4.  B1 Hq32 S1024 D128 (2 of 8) 21.5 / 26.4 / 50; 18.4 / 30.5 / 59; 20.0 / 35.6 / 70.
+struct SingleTiles {
+    long long n, heads, sms;  // query tiles of a head; heads of the batch
+    // The launches in question: as pairs they take as long as the longest one (with so few items the SMs' share of the key blocks
+    // never bounds them), and that is longer than all tiles on their own take: as long as the longest of them, or the SMs' share and a
+    // sixth for what list scheduling leaves over.  (Launches of more heads would end sooner in one stream as well, B1 Hq10 S4096 D128 in 54 us instead
+    // of 67, but take longer in several, 93 instead of 80 and 179 instead of 152, and stay pairs.)
+    bool bound_by_longest() const {
+        const long long blocks = heads * n * (n + 1) / 2, longest_pair = n % 2 == 0 ? 4 * n : std::max(4 * (n - 1), 3 * n);
+        return std::max(6 * n * sms, 7 * blocks) + 8 * sms < 2 * longest_pair * sms;
+    }
+    long long length(long long singles, long long place) const {
+        return place < singles ? 3 * (n - place) + 2 : 4 * (n - singles - 2 * (place - singles)) + 3;
+    }
+    long long time(long long singles) const {  // an even number of tiles in pairs
+        const long long places = singles + (n - singles) / 2, items = heads * places;
+        long long t = std::max(length(singles, 0), singles < places ? length(singles, singles) : 0);
+        if (items <= sms) return t;
+        for (long long place = sms / heads; place < places; ++place) {  // the last of the heads' items there: it has the longest one to wait for
+            const long long behind = (place + 1) * heads - 1 - sms;
+            if (behind >= 0) t = std::max(t, length(singles, place) + (behind < sms ? length(singles, (sms - 1 - behind) / heads) : t));
+        }
+        return t;
+    }
+    int count() const {
+        if (!bound_by_longest()) return 0;
+        long long singles = (n + 4) / 4;  // from here on the longest pair is no longer than the longest tile
+        singles += (n - singles) % 2;
+        long long best = singles, best_time = time(singles);
+        while ((singles -= 2) > 0 && length(singles, singles) <= best_time) {
+            const long long t = time(singles);
+            if (t <= best_time) best = singles, best_time = t;
+        }
+        return (int)best;
+    }
+};
 
 template <int D>
 int launch_fwd_t(const void* Q, const void* K, const void* V, void* O, float* LSE, const Shape& s, unsigned int* status,
@@ -676,8 +716,8 @@ int launch_fwd_t(const void* Q, const void* K, const void* V, void* O, float* LS
     p.cu = s.cu_seqlens;
     // Two query tiles per item share the K/V blocks and keep the tensor core busy in turns: 3 130 cycles per key block for both,
     // against 2 450 for one tile alone.  One tile per item finishes sooner when every tile gets an SM of its own (B200, D = 128
-    // causal: 128 tiles, B1 Hq16 S1024, 22.5 us as single tiles against 25.6 us as pairs) and when the longest item bounds the
-    // launch (single_tiles()).
+    // causal: 128 tiles, B1 Hq16 S1024, 22.5 us as single tiles against 25.6 us as pairs; with four streams 36 against 25 per launch
+    // of one); the longest ones also where they bound a launch of more tiles (SingleTiles).
     const int n_tiles = ((s.cu_seqlens ? s.max_seqlen : s.S) + kTile - 1) / kTile, n_seqs = s.cu_seqlens ? s.n_seqs : s.B;
     // Items of a packed batch are listed where that pays and the lengths differ (equal ones are in order as they are: with the
     // list 8 sequences of 300 tokens, Hq16 D128, take 18.4 us instead of 17.3).  Every sequence ends with one partial item at
@@ -694,16 +734,19 @@ int launch_fwd_t(const void* Q, const void* K, const void* V, void* O, float* LS
     // B1 Hq16 S4096 D128 94.0 -> 65.0, D64 82.2 -> 55.3; B1 Hq32 S2048 D128 71.9 -> 51.5; B16 Hq16 Hkv2 S4096 D64 (34 MB of K and
     // V) 764 -> 737, but B8 Hq32 Hkv8 S8192 D128 (268 MB) 3 968 -> 4 130.
     p.tile_slow = s.causal && !s.cu_seqlens && s.kv_rows() * s.D * 4 <= kOrderKvBytes;
-    p.tiles = items(1) <= sm_count() || (p.tile_slow && single_tiles(n_tiles, (long long)n_seqs * s.Hq, sm_count())) ? 1 : 2;
-    p.n_groups = (n_tiles + p.tiles - 1) / p.tiles;
+    p.tiles = items(1) <= sm_count() ? 1 : 2;
+    p.singles = p.tiles == 2 && p.tile_slow ? SingleTiles{n_tiles, (long long)n_seqs * s.Hq, sm_count()}.count() : 0;
+    p.n_groups = p.singles + (n_tiles - p.singles + p.tiles - 1) / p.tiles;
     p.scale_log2 = s.scale * kLog2e;
     const dim3 grid = p.n_listed    ? dim3((unsigned)items(p.tiles))
                       : p.tile_slow ? dim3(s.Hq, n_seqs, p.n_groups)
                                     : dim3(p.n_groups, s.Hq, n_seqs);
-    const bool more = items(p.tiles) > sm_count();
+    const bool more = (p.n_listed ? items(p.tiles) : (long long)p.n_groups * s.Hq * n_seqs) > sm_count();
     auto pick = [&](auto form) {
         constexpr Form F = decltype(form)::value;
-        return more ? gqa_fwd_sm100_kernel<D, F, true> : gqa_fwd_sm100_kernel<D, F, false>;
+        constexpr bool kCanStandAlone = F != kPacked;
+        if (kCanStandAlone && p.singles > 0) return more ? gqa_fwd_sm100_kernel<D, F, true, kCanStandAlone> : gqa_fwd_sm100_kernel<D, F, false, kCanStandAlone>;
+        return more ? gqa_fwd_sm100_kernel<D, F, true, false> : gqa_fwd_sm100_kernel<D, F, false, false>;
     };
     auto kernel = s.cu_seqlens ? pick(std::integral_constant<Form, kPacked>{})
                   : padded_form(s) ? pick(std::integral_constant<Form, kPadded>{})

@@ -3,6 +3,8 @@ not started (several per SM here), with rings and barrier phases running on; ite
 tile is missing or holds one row, the line between one and two query tiles per item, packed batches with items to pass
 over.  Parity per (sequence, KV head) against fp32 attention; tolerances are the common ones of the forward (bf16 P and
 O)."""
+import statistics
+
 import pytest
 import torch
 
@@ -82,25 +84,74 @@ def test_bits_do_not_depend_on_the_launch(gqa_lib, Hq, Hkv, S, D, causal):
     ops.check_status()
 
 
-@pytest.mark.parametrize("Hq,Hkv,S,D", [
-    (24, 8, 1000, 128),   # 192 single tiles: the longest item bounds the launch
-    (28, 4, 1024, 64),    # 224
-    (36, 6, 1024, 64),    # 288 tiles in pairs: one head more than the line allows
-    (24, 8, 900, 80),     # the last tile holds four rows
-    (64, 8, 600, 128),    # an odd number of tiles, the last one partial
-    (5, 1, 5000, 128),    # 200 single tiles, 40 key blocks in the longest
+@pytest.mark.parametrize("B,Hq,Hkv,S,D", [
+    (2, 12, 4, 1000, 128),  # the last 4 of a head's 8 tiles are items of their own, the others pairs; one item per SM at the most
+    (1, 28, 4, 1024, 64),   # 2 of 8
+    (1, 32, 8, 1024, 128),  # 2 of 8: as many heads as the line allows; 160 items
+    (1, 33, 11, 1024, 128), # pairs: one head more
+    (4, 10, 2, 700, 80),    # 2 of 6; the last tile is partial; padded head dimension
+    (1, 17, 1, 1600, 128),  # 5 of 13: an odd number of tiles
+    (1, 23, 23, 1300, 40),  # 3 of 11; the last tile holds 20 rows
+    (2, 32, 8, 600, 128),   # pairs, an odd number of tiles: the last one alone
+    (1, 5, 1, 5000, 128),   # 12 of 40
 ])
-def test_single_tiles_and_pairs_are_the_same_bits(gqa_lib, Hq, Hkv, S, D):
-    """Causal launches of more tiles than SMs on both sides of the line between one and two query tiles per item."""
+def test_single_tiles_and_pairs_are_the_same_bits(gqa_lib, B, Hq, Hkv, S, D):
+    """Causal launches of more tiles than SMs on both sides of the line between pairs of query tiles and the longest ones alone,
+    against one head at a time, where every tile gets an SM of its own."""
     gen = torch.Generator(device="cuda").manual_seed(12)
-    q, k, v = (torch.randn(1, h, S, D, generator=gen, device="cuda").bfloat16() for h in (Hq, Hkv, Hkv))
-    o, lse = ops.gqa_forward(q, k, v, causal=True)
-    G = Hq // Hkv
-    for h in range(Hkv):  # a head's shard: every tile gets an SM of its own
-        r = slice(h * G, (h + 1) * G)
-        o_h, lse_h = ops.gqa_forward(q[:, r].contiguous(), k[:, h:h + 1].contiguous(), v[:, h:h + 1].contiguous(), causal=True)
-        assert torch.equal(o_h, o[:, r]) and torch.equal(lse_h, lse[:, r]), h
+    q, k, v = (torch.randn(B, h, S, D, generator=gen, device="cuda").bfloat16() for h in (Hq, Hkv, Hkv))
+    o, lse = torch.full_like(q, float("nan")), torch.full((B, Hq, S), float("nan"), device="cuda")
+    ops.gqa_forward(q, k, v, causal=True, out=o, lse=lse)
+    for b in range(B):
+        for h in range(Hq):
+            g = h // (Hq // Hkv)
+            o_h, lse_h = ops.gqa_forward(q[b:b + 1, h:h + 1].contiguous(), k[b:b + 1, g:g + 1].contiguous(),
+                                         v[b:b + 1, g:g + 1].contiguous(), causal=True)
+            assert torch.equal(o_h[0, 0], o[b, h]) and torch.equal(lse_h[0, 0], lse[b, h]), (b, h)
     ops.check_status()
+
+
+def test_single_tiles_cost_four_streams_little(gqa_lib):
+    """Causal forwards of 32 heads end sooner alone with the longest tiles as items of their own; of 33 heads they are pairs.  Four
+    streams that fill the chip pay for the SMs' time: 1.19 times as much with the longest two of eight tiles alone, 1.41 times
+    with all eight alone.  The bound lies between."""
+    calls, S, D = 8, 1024, 128
+    streams = [torch.cuda.Stream() for _ in range(4)]
+
+    def captured(heads):
+        problems = []
+        for _ in streams:
+            q, k, v = (torch.randn(1, h, S, D, device="cuda").bfloat16() for h in (heads, 1, 1))
+            problems.append((q, k, v, torch.empty_like(q), torch.empty(1, heads, S, device="cuda")))
+        ops.gqa_forward(*problems[0][:3], causal=True)  # first use of the kernel, outside the capture
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            cur = torch.cuda.current_stream()
+            for s, (q, k, v, o, lse) in zip(streams, problems):
+                s.wait_stream(cur)
+                with torch.cuda.stream(s):
+                    for _ in range(calls):
+                        ops.gqa_forward(q, k, v, causal=True, out=o, lse=lse)
+            for s in streams:
+                cur.wait_stream(s)
+        return graph, problems
+
+    def ms(graph):
+        times = []
+        for _ in range(9):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            graph.replay()
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return statistics.median(times)
+
+    alone, pairs = captured(32), captured(33)
+    ms(pairs[0])
+    ratio = 33 / 32 * ms(alone[0]) / ms(pairs[0])
+    assert ratio <= 1.30, ratio
 
 
 @pytest.mark.parametrize("causal", [False, True])
