@@ -95,3 +95,127 @@ def test_separate_dq_at_tile_edges(gqa_lib, oracle, S, D, causal, layout):
     dq1, dk1, dv1 = ops.gqa_backward(tq, tk, tv, to, over, tlse, dq=over, dq_separate=True, **kw)
     ops.check_status(ws)
     assert torch.equal(dq1, dq) and torch.equal(dk1, dk) and torch.equal(dv1, dv)
+
+
+# Shapes whose main kernel takes much longer than the pass beside it: one KV head, so few KV tiles with all query heads each,
+# while the pass has a thread block per query tile.
+OUTLASTING = [(1, 8, 1, 1024, 64, True), (1, 8, 1, 1024, 128, False), (2, 6, 1, 700, 80, True)]
+
+
+def _problems(n, B, Hq, Hkv, S, D, causal):
+    """n problems as (inputs, expected gradients); the expected ones from calls with the host waiting before and after each."""
+    gen = torch.Generator(device="cuda").manual_seed(41)
+    out = []
+    for _ in range(n):
+        q, k, v, do = (torch.randn(B, h, S, D, generator=gen, device="cuda").bfloat16() for h in (Hq, Hkv, Hkv, Hq))
+        o, lse = ops.gqa_forward(q, k, v, causal=causal)
+        ws = torch.empty(ops.bwd_workspace_bytes(B, Hq, Hkv, S, D, causal), dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        want = ops.gqa_backward(q, k, v, o, do, lse, causal=causal, workspace=ws, dq_separate=True)
+        torch.cuda.synchronize()
+        ops.check_status(ws)
+        out.append(((q, k, v, o, do, lse), want))
+    return out
+
+
+def _call_and_consume(inputs, ws, grads, results, causal):
+    """The backward; directly behind it a reader of all it writes and a writer of all it reads (copies that later calls do not
+    use): kernels that come too early if the call's last kernel does not wait for the main kernel."""
+    q, k, v, o, do, lse = inputs
+    ops.gqa_backward(q, k, v, o, do, lse, causal=causal, workspace=ws, dq_separate=True, dq=grads[0], dk=grads[1], dv=grads[2])
+    for r, g in zip(results, grads):
+        r.copy_(g)
+    for g in grads:
+        g.zero_()
+    for t in (q, k, v, do):
+        t.fill_(float("nan"))
+
+
+@pytest.mark.parametrize("case", OUTLASTING)
+def test_separate_dq_keeps_the_order_of_the_stream(gqa_lib, case):
+    """Calls one behind the other on one workspace and one set of gradients, with no wait on the host: eagerly, from a captured graph
+    and on two streams at once with a workspace each."""
+    B, Hq, Hkv, S, D, causal = case
+    n = 6
+    problems = _problems(n, *case)
+    results = [[torch.empty_like(g) for g in want] for _, want in problems]
+    n_ws = ops.bwd_workspace_bytes(B, Hq, Hkv, S, D, causal)
+    lanes = [(torch.cuda.Stream(), torch.empty(n_ws, dtype=torch.uint8, device="cuda"), [torch.empty_like(g) for g in problems[0][1]])
+             for _ in range(2)]  # stream, workspace, gradients
+    work = [[t.clone() for t in inputs] for inputs, _ in problems]
+
+    def refill():
+        for w, (inputs, _) in zip(work, problems):
+            for dst, src in zip(w, inputs):
+                dst.copy_(src)
+        for r in results:
+            for t in r:
+                t.fill_(float("nan"))
+
+    def check(what):
+        torch.cuda.synchronize()
+        for _, ws, _ in lanes:
+            ops.check_status(ws)
+        for i, (r, (_, want)) in enumerate(zip(results, problems)):
+            for name, a, b in zip(("dQ", "dK", "dV"), r, want):
+                assert torch.equal(a, b), (what, i, name)
+
+    def run(streams):
+        for i in range(n):
+            st, ws, grads = lanes[i % len(streams)]
+            with torch.cuda.stream(streams[i % len(streams)]):
+                _call_and_consume(work[i], ws, grads, results[i], causal)
+
+    lanes[0][1].fill_(255)
+    lanes[1][1].zero_()  # not used by the first runs: its status word reads as no report
+    for trial in range(3):
+        refill()
+        torch.cuda.synchronize()
+        run([lanes[0][0]])
+        check(("one stream", trial))
+    for trial in range(3):
+        refill()
+        torch.cuda.synchronize()
+        run([lanes[0][0], lanes[1][0]])
+        check(("two streams", trial))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=lanes[0][0]):
+        run([lanes[0][0]])
+    for trial in range(3):
+        refill()
+        graph.replay()
+        check(("graph", trial))
+
+
+@pytest.mark.parametrize("D,causal", [(64, True), (128, False), (80, True)])
+def test_separate_dq_with_a_head_split(gqa_lib, D, causal):
+    """A split that takes effect puts the sum of the parts between the two kernels: dK and dV are the bits of the split alone, dQ
+    the bits of the separate pass alone."""
+    B, Hq, Hkv, S = 1, 8, 1, 1000
+    n_ws = ops.bwd_workspace_bytes(B, Hq, Hkv, S, D, causal, split_heads=True)
+    assert n_ws > ops.bwd_workspace_bytes(B, Hq, Hkv, S, D, causal)
+    ((q, k, v, o, do, lse), want), = _problems(1, B, Hq, Hkv, S, D, causal)
+    ws = torch.full((n_ws,), 255, dtype=torch.uint8, device="cuda")
+    _, dk0, dv0 = ops.gqa_backward(q, k, v, o, do, lse, causal=causal, workspace=ws, split_heads=True)
+    for _ in range(3):
+        dq, dk, dv = ops.gqa_backward(q, k, v, o, do, lse, causal=causal, workspace=ws, split_heads=True, dq_separate=True)
+        got = [t.clone() for t in (dq, dk, dv)]  # directly behind the call
+        ops.check_status(ws)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], dk0) and torch.equal(got[2], dv0)
+
+
+@pytest.mark.parametrize("S,over", [(128, "q"), (128, "k"), (128, "v"), (100, "k"), (500, "q"), (1024, "do")])
+@pytest.mark.parametrize("D", [64, 128])
+def test_separate_dq_in_place_of_an_input(gqa_lib, S, over, D):
+    """dQ written over an input of its own size is the same bits: over Q and dO, whose rows only their own thread block reads, at any
+    length; over K and V where one query tile sees one key block."""
+    B, H = 3, 4
+    ((q, k, v, o, do, lse), want), = _problems(1, B, H, H, S, D, False)
+    ws = torch.full((ops.bwd_workspace_bytes(B, H, H, S, D),), 255, dtype=torch.uint8, device="cuda")
+    t = {"q": q, "k": k, "v": v, "do": do}
+    t[over] = t[over].clone()
+    dq, dk, dv = ops.gqa_backward(t["q"], t["k"], t["v"], o, t["do"], lse, workspace=ws, dq=t[over], dq_separate=True)
+    got = [x.clone() for x in (dq, dk, dv)]
+    ops.check_status(ws)
+    for name, a, b in zip(("dQ", "dK", "dV"), got, want):
+        assert torch.equal(a, b), name
