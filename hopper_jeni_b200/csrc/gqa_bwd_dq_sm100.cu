@@ -21,8 +21,13 @@
 // registers: while the warpgroups work on block n the issuer produces dP(n+1) and S(n+1).  Per block of D = 128 the products
 // take 1 650 cycles (two of 128 x 128 x 128 and the 78 cycles of a K step with A in TMEM) and the exponentials 1 024.
 //
-// The kernel is launched behind the main kernel and runs beside it on the SMs that it leaves idle.  B200, whole call, us, one
-// after the other with blocks of 64 keys and two warpgroups -> now: B2 Hq16 Hkv4 S1024 causal D64 77.7 -> 53.6, D80 105 -> 71.6,
+// The kernel is launched behind the main kernel and runs beside it on the SMs that it leaves idle.  It is the one dependent launch
+// that does not wait for the kernel in front before it touches global memory.  What makes that safe: the main kernel's
+// trigger stands behind its wait for the preprocess kernel and behind its release of `prep_seen`; nothing is launched between the
+// two; dQ overlaps nothing that the main kernel reads (the host looks); the shared memory of both keeps their blocks off one another's
+// SMs.
+//
+// B200, whole call, us, one after the other with blocks of 64 keys and two warpgroups -> now: B2 Hq16 Hkv4 S1024 causal D64 77.7 -> 53.6, D80 105 -> 71.6,
 // D128 109 -> 78.9; B1 Hq32 Hkv8 S2048 D128 279 -> 254; B1 Hq64 Hkv8 S4096 D128 causal 1 123 -> 1 023.  (Accumulated dQ: 60.4,
 // 79.1, 90.8, 174, 780.)
 //
@@ -62,7 +67,8 @@ struct DqCfg {
     static constexpr uint32_t kColS = 0, kColDP = 256, kColDQ = 384;  // S: two buffers of 128 columns
     static_assert(kColDQ + D <= 512, "TMEM budget");
     static_assert(kSmemTotal <= 227 * 1024, "shared memory budget");
-    static_assert(kSmemTotal > 114 * 1024, "one CTA per SM is assumed by the 512-column TMEM allocation");
+    // (nor beside a block of the main kernel, which may not have taken its tensor memory yet when this one comes up)
+    static_assert(kSmemTotal > kHalfSharedMemory, "one CTA per SM is assumed by the 512-column TMEM allocation");
 };
 
 struct DqParams {

@@ -170,7 +170,7 @@ struct BwdCfg {
     static_assert(kColDK + D + (kPAliasesS ? 0 : 64) <= 512, "TMEM budget");
     static constexpr int kOffList = kSmemTotal;  // packed batches: the work list
     static_assert(kOffList % alignof(PackedList) == 0 && kSmemTotal + (int)sizeof(PackedList) <= 227 * 1024, "shared memory budget");
-    static_assert(kSmemTotal > 114 * 1024, "one CTA per SM is assumed by the 512-column TMEM allocation");
+    static_assert(kSmemTotal > kHalfSharedMemory, "one CTA per SM is assumed by the 512-column TMEM allocation");
 };
 
 struct BwdParams {
@@ -415,7 +415,8 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
     if constexpr (!kWithDQ) {
         // The separate dQ pass comes up beside this kernel, on the SMs that it leaves idle, and reads what the preprocess
         // kernel wrote: `prep_seen` hands that on (this thread has seen it, the pass acquires the word).  Every block is
-        // resident by then, and none waits for the pass.
+        // resident by then, and none waits for the pass.  The pass does not wait for this kernel before it begins, so the trigger stays
+        // behind pdl_wait() and the release, in this order.
         if (tid == 0) {
             if (blockIdx.x == 0) st_release_gpu(p.prep_seen, 1u);
             pdl_launch_dependents();
@@ -613,7 +614,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
             if (idx < 0) break;
             const int n_iter = decode(idx).n_iter;
             ok = mbar_wait(kv_full, j & 1, ctx, 20);
-            if (kOrdered && j > 0) ok = ok && mbar_wait(acc_empty, (j - 1) & 1, ctx, 37);
+            if (kOrdered && j > 0) ok = ok && mbar_wait(acc_empty, (j - 1) & 1, ctx, 37);  // (launched with one item per block it has no j > 0)
             for (int it = 0; it < n_iter && ok; ++it, ++gi) {
                 const int qs = gi % Cfg::kQStages, dos = gi % Cfg::kDOStages;
                 ok = mbar_wait(&q_full[qs], (gi / Cfg::kQStages) & 1, ctx, 21);
@@ -771,7 +772,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
         uint8_t* stage = sDQ + warp * kWarpStage + lane * 128;
         const int sw = lane & 7;
         // The loop exists twice, with and without the deterministic mode's bookkeeping (the `det` tag below): the role
-        // is short of registers, and the default path should not carry the turn state.
+        // is short of registers, and the default path should not carry the turn state.  (See the end of the role.)
         auto drain_items = [&](auto det) {
         constexpr bool kDet = decltype(det)::value;
         // Deterministic mode: the reductions into one 32-row slice of the accumulator are applied in the order of the item
@@ -839,7 +840,6 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
             if (!mbar_wait(dq_full, gi & 1, ctx, 40)) { going = false; break; }  // dQ(it) complete
             tc_fence_after_sync();
             GQA_TRACE(2, gi, 0);
-            constexpr int kRounds = D / (32 * Cfg::kDqBoxes);
             if constexpr (Cfg::kDrainEarlyRelease) {
                 static_assert(!Cfg::kDrainEarlyRelease || (D == 128 && Cfg::kDqBoxes == 1), "four 32-column chunks, one box");
                 auto fill_box = [&](const uint32_t (&v)[32]) {
@@ -897,6 +897,7 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                 }
                 if (kDet && turn_mine) pending = true;
             } else {
+                constexpr int kRounds = D / (32 * Cfg::kDqBoxes);
     #pragma unroll 1
                 for (int rnd = 0; rnd < kRounds; ++rnd) {
                     // (Plain stores whose order against the TMEM loads is left to the compiler.  Measured alternatives,
@@ -948,8 +949,10 @@ gqa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
         if (warp == 0) GQA_MARK(7);
         count_reduced();
         };
-        // (The default form keeps the ordered loop, which it never takes: with the unordered one alone ptxas schedules the role so
-        // that B2 Hq32 S1537 D128 takes 170 us instead of 166 and B4 Hq32 S1024 D128 143 instead of 140.)
+        // Every form holds both loops, and takes the one that is its own: the host gives turns to the ordered forms and to no other,
+        // since only they have a warp that hands them on.  With one loop each, ptxas 12.9.86 schedules the role so that default
+        // calls take longer (B200, us: B2 Hq32 S1537 D128 causal 160 -> 167, B4 Hq32 S1024 D128 causal 138.5 -> 142.5, packed D64 122.5 -> 128,
+        // packed D128 197 -> 194.5) and ordered ones too (B16 Hq16 Hkv2 S2048 D64 causal 627 -> 635).
         if (p.dq_turn)
             drain_items(std::true_type{});
         else
@@ -1261,6 +1264,8 @@ int launch_bwd_t(const void* Q, const void* K, const void* V, const void* dO, co
     }
     const bool varlen = s.cu_seqlens != nullptr;
     if (varlen && (!dq_accum || dq_turn || parts != 1 || !s.bshd || s.B != 1)) return GQA_ERR_BAD_ARGUMENT;
+    if (dq_turn && !dq_accum) return GQA_ERR_BAD_ARGUMENT;
+    // (p.dq_turn below is set for the ordered forms and for no other: see the end of the drain role)
     auto kernel = varlen      ? gqa_bwd_sm100_kernel<D, true, true, false, false>
                   : !dq_accum ? (padded_form(s) ? gqa_bwd_sm100_kernel<D, false, false, true, false> : gqa_bwd_sm100_kernel<D, false, false, false, false>)
                   : dq_turn   ? (padded_form(s) ? gqa_bwd_sm100_kernel<D, true, false, true, true> : gqa_bwd_sm100_kernel<D, true, false, false, true>)

@@ -41,8 +41,11 @@ int make_tile3_tmap(CUtensorMap* out, const void* base, uint64_t cols, uint64_t 
 int make_f32box3_tmap(CUtensorMap* out, const void* base, uint64_t cols, uint64_t S, uint64_t n_outer, uint32_t box_rows);
 int make_col8_3_tmap(CUtensorMap* out, const void* base, uint64_t S, uint64_t n_outer, uint32_t box_rows);
 
+// Half of an SM's shared memory: of kernels whose blocks take more, an SM holds one block at a time.
+constexpr int kHalfSharedMemory = 114 * 1024;
+
 // Launch whose blocks may start before the kernel in front of it in the stream has ended: the kernel must call pdl_wait()
-// (sm100_ptx.cuh) before it touches global memory.
+// (sm100_ptx.cuh) before it touches global memory.  The one exception is the separate dQ pass, which says why it may.
 template <class... P, class... A>
 cudaError_t launch_after(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, A&&... args) {
     cudaLaunchAttribute attr;

@@ -71,7 +71,7 @@ struct FwdCfg {
     static constexpr uint32_t kColS0 = 0, kColS1 = 128, kColO0 = 256, kColO1 = 256 + D;
     static_assert(256 + 2 * D <= 512, "TMEM budget");
     static_assert(kOffList % alignof(PackedList) == 0 && kSmemTotal + (int)sizeof(PackedList) <= 227 * 1024, "shared memory budget");
-    static_assert(kSmemTotal > 114 * 1024, "one CTA per SM is assumed by the 512-column TMEM allocation");
+    static_assert(kSmemTotal > kHalfSharedMemory, "one CTA per SM is assumed by the 512-column TMEM allocation");
 };
 
 struct FwdParams {

@@ -51,12 +51,13 @@ struct BwdWorkspace {
     }
 };
 
-// Stage 1 of the backward: Delta = rowsum(dO*O); with `delta` it is stored as fp32, with the column arrays
-// the bf16 splits of -LSE*inv_scale and -Delta are stored (16 bytes per row each) and, if given, the dQ
-// accumulator is zeroed.
 // Words of the 256 bytes in front of the workspace, all zeroed by the preprocess kernel: the status, the main kernel's work
 // counter, and whether the main kernel has seen what the preprocess kernel wrote (for the separate dQ pass beside it).
 constexpr int kWorkCounterWord = 16, kPrepSeenWord = 32;
+
+// Stage 1 of the backward: Delta = rowsum(dO*O); with `delta` it is stored as fp32, with the column arrays
+// the bf16 splits of -LSE*inv_scale and -Delta are stored (16 bytes per row each) and, if given, the dQ
+// accumulator is zeroed.
 // `status` (the 256 bytes in front of the workspace) and the `n_turns` words at `turns` are zeroed as well.
 // `S_bshd` / `H_bshd`: 0 when O, dO are in [B,H,S,D] order, else S and Hq of the [B,S,H,D] layout they are in.
 int launch_bwd_preprocess(const void* O, const void* dO, const float* lse, float inv_scale, float* delta,
@@ -90,8 +91,9 @@ int launch_bwd_main_sm100(const void* Q, const void* K, const void* V, const voi
                           const void* delta_cols, float* dq_accum, unsigned int* dq_turn, void* dK, void* dV,
                           const Shape& s, unsigned int* status, int parts, float* partial, cudaStream_t stream);
 // The alternative dQ path: a separate query-parallel pass that recomputes S and dP and writes dQ once (no accumulator,
-// no finalise, bit-reproducible).  `delta` is rowsum(dO * O) as fp32 per query row.  `beside`: it follows the main kernel's
-// launch directly and may run beside it; else it starts when everything in front of it has ended.
+// no finalise, bit-reproducible).  `delta` is rowsum(dO * O) as fp32 per query row.  `beside`: it follows directly on the launch of
+// the main kernel without its dQ part, dQ overlaps nothing that one reads, and it may run beside it; else it starts when everything in
+// front of it has ended.
 int launch_bwd_dq_sm100(const void* Q, const void* K, const void* V, const void* dO, const float* lse,
                         const float* delta, void* dQ, const Shape& s, unsigned int* status, bool beside,
                         cudaStream_t stream);

@@ -28,7 +28,7 @@ __device__ __forceinline__ uint2 split3_bf16(float x) {
                       (uint32_t)__bfloat16_as_ushort(lo));
 }
 
-constexpr int kStatusWords = 64;  // the status word and the work counter behind it: 256 bytes
+constexpr int kStatusWords = 64;  // the 256 bytes in front of the workspace (kWorkCounterWord, kPrepSeenWord)
 
 // (The words that the backward needs zeroed ride along: as memset nodes in front they were a launch each.)
 // One group of D/8 lanes per row; each lane owns 8 consecutive elements (one 16-byte load

@@ -180,7 +180,8 @@ __device__ __forceinline__ void st_release_cta(uint32_t* p, uint32_t v) {
 // ----------------------------------------------------------------------------
 // Programmatic dependent launch.  A kernel launched with launch_after() (gqa_common.cuh) may start while the one before it
 // in the stream still runs, once every block of that one has called pdl_launch_dependents() or ended; pdl_wait() returns when
-// that one has completed and its writes are visible.  Nothing it wrote, and nothing it may still read, is touched before.
+// that one has completed and its writes are visible.  Nothing it wrote, and nothing it may still read, is touched before (but for
+// the separate dQ pass: see gqa_bwd_dq_sm100.cu).
 // ----------------------------------------------------------------------------
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
