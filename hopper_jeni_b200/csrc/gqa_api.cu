@@ -172,10 +172,9 @@ int run_bwd(const void* Q, const void* K, const void* V, const void* O, const vo
     float* dq_accum = reinterpret_cast<float*>(w + ws.dq_accum_off);
     float* delta_f32 = reinterpret_cast<float*>(w + ws.delta_f32_off);
     // The dQ path.  Default: fp32 TMA reduce-add of the main kernel's dQ tiles into the accumulator: measured faster
-    // than the separate query-parallel pass wherever the KV tiles fill the chip (1.3-1.7x).  Where they leave more than half of
-    // the SMs idle the separate pass, beside the main kernel, takes 0.8 to 0.93 of the default's time in one stream, but 1.3 to
-    // 1.6 of it in four streams that fill the chip together (it does half as many products again), so it is taken only when
-    // asked for.
+    // than the separate query-parallel pass wherever the KV tiles fill the chip.  Where they leave many SMs idle the separate pass,
+    // beside the main kernel, is faster in one stream and slower in several that fill the chip together (it does half as many
+    // products again), so it is taken only when asked for (figures: GQA_BWD_DQ_SEPARATE in gqa.h).
     const bool dq_separate = (flags & GQA_BWD_DQ_SEPARATE) != 0;
     unsigned int* dq_turn = nullptr;
     if ((flags & GQA_BWD_DETERMINISTIC) && !dq_separate) dq_turn = reinterpret_cast<unsigned int*>(w + ws.dq_turn_off);

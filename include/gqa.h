@@ -126,9 +126,11 @@ int gqa_bwd(const void* Q, const void* K, const void* V, const void* O, const vo
  * over the key tiles, as the reference's first generations do, src/attention/GQA_bwd.cu:29, :415, :1416) instead
  * of accumulating the main kernel's dQ tiles with fp32 reductions.  S and dP are then computed twice, but dQ needs
  * no accumulator, no finalise pass, and is bit-reproducible by construction.  Measured 1.3-1.7x slower than the
- * default where the KV tiles (B * Hkv * ceil(S / 128)) fill the chip.  It runs on the SMs that they leave idle: with fewer
- * than 50 of them, or 100 with a causal mask, a call takes 0.80 to 0.95 of the default's time, if no other stream wants
- * those SMs.  No mode selects it by itself.  Same workspace size.
+ * default where the KV tiles (B * Hkv * ceil(S / 128)) fill the chip.  It runs on the SMs that they leave idle: with up to
+ * 40 KV tiles, or 64 with a causal mask, a call that has the GPU to itself takes 0.78 to 0.95 of the default's time (560 shapes
+ * on a B200; with 56, or 104 with a causal mask, 0.82 to 1.19, by shape).  Streams that fill the GPU together lose with
+ * it: four take 1.3 to 1.65 times as long as with the default.  No mode selects it by itself.  Same workspace size.
+ * dQ may be written over Q or dO.
  */
 #define GQA_BWD_DETERMINISTIC 1u
 #define GQA_BWD_SPLIT_HEADS 4u
