@@ -40,6 +40,7 @@ def test_deterministic_backward_matches_oracle(gqa_lib, oracle, shape, causal):
     (2, 4, 2, 333, 40),
     (1, 6, 2, 333, 80),     # the padded form
     (1, 8, 1, 129, 128),    # the second tile holds one row
+    (1, 2, 1, 1100, 64),    # nine tiles: four of them in descending order when causal, five more behind
 ])
 def test_ordered_form_matches_oracle_at_odd_sizes(gqa_lib, oracle, shape, causal):
     B, Hq, Hkv, S, D = shape
