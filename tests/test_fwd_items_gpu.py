@@ -108,6 +108,9 @@ def test_single_tiles_and_pairs_are_the_same_bits(gqa_lib, B, Hq, Hkv, S, D):
             o_h, lse_h = ops.gqa_forward(q[b:b + 1, h:h + 1].contiguous(), k[b:b + 1, g:g + 1].contiguous(),
                                          v[b:b + 1, g:g + 1].contiguous(), causal=True)
             assert torch.equal(o_h[0, 0], o[b, h]) and torch.equal(lse_h[0, 0], lse[b, h]), (b, h)
+    if D in (64, 128):
+        o_t, lse_t = ops.gqa_forward(*(t.transpose(1, 2).contiguous() for t in (q, k, v)), causal=True, layout="bshd")
+        assert torch.equal(o_t.transpose(1, 2), o) and torch.equal(lse_t, lse)
     ops.check_status()
 
 
